@@ -57,13 +57,13 @@ __global__ void normals_kernel(const float *__restrict__ pcd, int rows, int cols
     out[p * 3 + 2] = n.z;
 }
 
-// 16- and 8-byte asynchronous copies from global to shared memory (no
+// 16- and 4-byte asynchronous copies from global to shared memory (no
 // registers held while they are in flight).
 __device__ __forceinline__ void cp_async16(unsigned dst, const void *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(unsigned dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async4(unsigned dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
@@ -134,14 +134,18 @@ __device__ __forceinline__ float icp_float_of_fixed(__int128 t) {
 // getPoint are shared by its points, and its neighbours' points are
 // recomputed from their depths with the same roundings, so the three images
 // equal those of the three separate launches bit for bit. The source points
-// go out as float triples; the target point and normal of a pixel as one
-// 16-byte (x, y, z, nx) and one 8-byte (ny, nz) entry, the layout the
-// iteration kernel stages in shared memory, x holding NaN where the
-// reference's search skips the tap (py.z == 0, or n.x == 0 point-to-plane:
-// kokkosICP.cpp:89,100) so that its distance fails every comparison.
+// go out as float triples; a target pixel as one 16-byte entry, the layout
+// the iteration kernel stages in shared memory: point to point (x, y, z, 0),
+// x holding +infinity where the reference's search skips the tap (py.z == 0,
+// kokkosICP.cpp:89), so that its distance is infinite; point to plane
+// (z, nx, ny, nz), z holding NaN where the search skips it (py.z == 0 or
+// n.x == 0, :100), so that its distance fails every comparison. The x and y of
+// a point-to-plane tap are its z times its column's and row's quotient (the
+// roundings of getPoint), which go out as the table uv (cols, then rows): a
+// 16-byte entry instead of 24 bytes for the point and the normal.
 __global__ void icp_prep_kernel(const uint16_t *__restrict__ d1, const uint16_t *__restrict__ d2, int rows, int cols,
                                 Intr in, int type, float *__restrict__ xp, float4 *__restrict__ ya,
-                                float2 *__restrict__ yb, IcpInit ini, IcpState *__restrict__ st) {
+                                float *__restrict__ uv, IcpInit ini, IcpState *__restrict__ st) {
     if (blockIdx.x == 0 && blockIdx.y == 0) {  // the call's state: Txy, identity best, counters cleared
         const int t = threadIdx.x;
         if (t < 16) {
@@ -162,6 +166,8 @@ __global__ void icp_prep_kernel(const uint16_t *__restrict__ d1, const uint16_t 
     if (j >= cols || i >= rows) return;
     const size_t p = (size_t)i * cols + j;
     const float qx = __fdiv_rn(__fsub_rn((float)j, in.cj), in.fx), qy = __fdiv_rn(__fsub_rn((float)i, in.ci), in.fy);
+    if (i == 0) uv[j] = qx;
+    if (j == 0) uv[cols + i] = qy;
     auto pt = [](float ux, float uy, float d) { return F3{__fmul_rn(ux, d), __fmul_rn(uy, d), d}; };
     const F3 x = pt(qx, qy, depth_m(__ldg(d1 + p)));
     const F3 c = pt(qx, qy, depth_m(__ldg(d2 + p)));
@@ -184,9 +190,10 @@ __global__ void icp_prep_kernel(const uint16_t *__restrict__ d1, const uint16_t 
             n = f3normalized(f3add(f3add(f3add(n1, n2), n3), n4));
         }
     }
-    const bool tap = c.z != 0 && (type == SS_ICP_POINT_TO_POINT || n.x != 0);
-    ya[p] = make_float4(tap ? c.x : __int_as_float(0x7fc00000), c.y, c.z, n.x);
-    yb[p] = make_float2(n.y, n.z);
+    if (type == SS_ICP_POINT_TO_POINT)
+        ya[p] = make_float4(c.z != 0 ? c.x : __int_as_float(0x7f800000), c.y, c.z, 0.f);
+    else
+        ya[p] = make_float4(c.z != 0 && n.x != 0 ? c.z : __int_as_float(0x7fc00000), n.x, n.y, n.z);
 }
 
 
@@ -404,27 +411,30 @@ __device__ __forceinline__ void fp2_add2(f32x2 &h, f32x2 &l, f32x2 h2, f32x2 l2)
     l = f2_sub(t, f2_sub(h, s));
 }
 
-// The CTA's 18 sums: each lane's pairs, a warp transpose-reduce (at offset o a
-// lane keeps the half of its values selected by lane bit o and adds the other
-// lane's; after offsets 16..1 lane v holds the warp's pair of value v), then
-// the warps' pairs by a fixed tree; thread v < kIcpSums returns the CTA's
-// pair of value v.
-__device__ __forceinline__ float2 icp_cta_sum(float *vh, float *vl, float2 (*red)[kIcpSums]) {
+// The CTA's 18 sums. Values 1..16 (a lane's pairs vh, vl): a warp
+// transpose-reduce (at offset o = 16, 8, 4, 2 a lane keeps the half of its
+// values selected by lane bit o and adds the other lane's, then lanes 2 v and
+// 2 v + 1 add their halves), 16 pair additions, two per paired instruction.
+// Values 0 and 17, the counts n_cors and n_x of the warp, are integers and
+// come as such. Then the warps' pairs by a fixed tree; thread v < kIcpSums
+// returns the CTA's pair of value v.
+constexpr int kIcpPairs = 16;  // values 1..16
+__device__ __forceinline__ float2 icp_cta_sum(float *vh, float *vl, int n_cors, int n_x, float2 (*red)[kIcpSums]) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        const bool upper = (lane & o) != 0;
-        if (o >= 2) {  // two values per step in paired instructions (the same roundings)
+    for (int h = kIcpPairs / 2; h >= 1; h >>= 1) {  // h values are kept; lane offset 2 h
+        const bool upper = (lane & (2 * h)) != 0;
+        if (h >= 2) {  // two values per step in paired instructions (the same roundings)
 #pragma unroll
-            for (int k = 0; k < o; k += 2) {
+            for (int k = 0; k < h; k += 2) {
                 float kh[2], kl[2], rh[2], rl[2];
 #pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    const float sh = upper ? vh[k + u] : vh[k + u + o], sl = upper ? vl[k + u] : vl[k + u + o];
-                    kh[u] = upper ? vh[k + u + o] : vh[k + u];
-                    kl[u] = upper ? vl[k + u + o] : vl[k + u];
-                    rh[u] = __shfl_xor_sync(0xffffffffu, sh, o);
-                    rl[u] = __shfl_xor_sync(0xffffffffu, sl, o);
+                    const float sh = upper ? vh[k + u] : vh[k + u + h], sl = upper ? vl[k + u] : vl[k + u + h];
+                    kh[u] = upper ? vh[k + u + h] : vh[k + u];
+                    kl[u] = upper ? vl[k + u + h] : vl[k + u];
+                    rh[u] = __shfl_xor_sync(0xffffffffu, sh, 2 * h);
+                    rl[u] = __shfl_xor_sync(0xffffffffu, sl, 2 * h);
                 }
                 f32x2 ph = f2_pack(kh[0], kh[1]), pl = f2_pack(kl[0], kl[1]);
                 fp2_add2(ph, pl, f2_pack(rh[0], rh[1]), f2_pack(rl[0], rl[1]));
@@ -434,13 +444,21 @@ __device__ __forceinline__ float2 icp_cta_sum(float *vh, float *vl, float2 (*red
         } else {
             const float sh = upper ? vh[0] : vh[1], sl = upper ? vl[0] : vl[1];
             float kh = upper ? vh[1] : vh[0], kl = upper ? vl[1] : vl[0];
-            const float rh = __shfl_xor_sync(0xffffffffu, sh, 1), rl = __shfl_xor_sync(0xffffffffu, sl, 1);
+            const float rh = __shfl_xor_sync(0xffffffffu, sh, 2), rl = __shfl_xor_sync(0xffffffffu, sl, 2);
             fp2_add(kh, kl, rh, rl);
             vh[0] = kh;
             vl[0] = kl;
         }
     }
-    if (lane < kIcpSums) red[wid][lane] = make_float2(vh[0], vl[0]);
+    {
+        const float rh = __shfl_xor_sync(0xffffffffu, vh[0], 1), rl = __shfl_xor_sync(0xffffffffu, vl[0], 1);
+        fp2_add(vh[0], vl[0], rh, rl);  // lanes 2 v, 2 v + 1: value 1 + v
+    }
+    if ((lane & 1) == 0) red[wid][1 + (lane >> 1)] = make_float2(vh[0], vl[0]);
+    if (lane == 0) {
+        red[wid][0] = make_float2((float)n_cors, 0.f);
+        red[wid][kIcpSums - 1] = make_float2((float)n_x, 0.f);
+    }
     __syncthreads();
     float h = 0.f, l = 0.f;
     if (threadIdx.x < kIcpSums) {  // the eight warps' pairs by a tree, three additions deep
@@ -459,10 +477,14 @@ __device__ __forceinline__ float2 icp_cta_sum(float *vh, float *vl, float2 (*red
 
 // Target pixels staged per CTA: a tile's 10 x 10 windows (kokkosICP.cpp:81-83)
 // usually fall inside a region of some 42 x 26 pixels; up to this many are
-// staged, larger regions are read from global memory.
+// staged, larger regions are read from global memory. A region holds at least
+// one window, so neither of its sides exceeds kIcpEdge.
 constexpr int kIcpStage = 1536;
+constexpr int kIcpEdge = 160;
+static_assert(kIcpEdge * 10 >= kIcpStage, "a staged region's sides fit the quotient tables");
 constexpr int kIcpSearch = 5;         // n_search (kokkosICP.cpp:53)
 constexpr float kIcpMaxDist = 0.075f; // max_dist (kokkosICP.cpp:55)
+constexpr int kIcpCoop = 8;           // up to this many windows of a warp are left to the whole warp, one at a time
 
 // The transformed source point px = Txy x and its window centre
 // (kokkosICP.cpp:72-76); true when the reference searches (x.z != 0 and the
@@ -480,20 +502,18 @@ __device__ __forceinline__ bool icp_center(const Mat34 &T, F3 x, Intr in, int ro
     return ci > kIcpSearch && ci < rows - kIcpSearch && cj > kIcpSearch && cj < cols - kIcpSearch;
 }
 
-// A tap's distance (kokkosICP.cpp:91,101-102) from its (x, y, z, nx) and
-// (ny, nz) entries; NaN for a tap the reference skips.
-template <int kType>
-__device__ __forceinline__ float icp_tap_dist(const float4 a, const float2 b, F3 px) {
-    const F3 py{a.x, a.y, a.z};
-    return kType == SS_ICP_POINT_TO_POINT ? f3len(f3sub(py, px)) : fabsf(f3dot(f3sub(py, px), F3{a.w, b.x, b.y}));
+// A point-to-plane tap's point: its z times its column's and row's quotients
+// (getPoint's roundings); NaN in a tap the reference skips.
+__device__ __forceinline__ F3 icp_tap_point(const float4 a, float u, float v) {
+    return {__fmul_rn(u, a.x), __fmul_rn(v, a.x), a.x};
 }
 
-// The search state of one window: the even and the odd columns keep separate
-// minima (two independent compare chains) with their taps' indices (staged
-// or image indices, increasing in the window's scan order); the first tap of
-// the scan with the smallest distance is then the one of the smaller
-// minimum, on a tie the earlier tap. Starting from max_dist, the accepted
-// taps of `dist < smallest && dist < max_dist` are exactly those of
+// The search state of one point-to-plane window: the even and the odd columns
+// keep separate minima (two independent compare chains) with their taps'
+// indices (staged or image indices, increasing in the window's scan order);
+// the first tap of the scan with the smallest distance is then the one of the
+// smaller minimum, on a tie the earlier tap. Starting from max_dist, the
+// accepted taps of `dist < smallest && dist < max_dist` are exactly those of
 // `dist < min(smallest, max_dist)`.
 struct IcpBest {
     float s0 = kIcpMaxDist, s1 = kIcpMaxDist;
@@ -512,94 +532,290 @@ struct IcpBest {
     __device__ __forceinline__ int best() const { return (s1 < s0 || (s1 == s0 && b1 < b0)) ? b1 : b0; }
 };
 
-// The distances of one tap to two transformed source points (packed x, y and
-// z of both): icp_tap_dist for each, the same roundings in the same order.
-template <int kType>
-__device__ __forceinline__ void icp_tap_dist2(const float4 a, const float2 b, f32x2 px, f32x2 py, f32x2 pz, float &da,
-                                              float &db) {
-    const f32x2 dx = f2_sub(f2_pack(a.x, a.x), px), dy = f2_sub(f2_pack(a.y, a.y), py),
-                dz = f2_sub(f2_pack(a.z, a.z), pz);
-    if (kType == SS_ICP_POINT_TO_POINT) {
-        f2_unpack(f2_add(f2_add(f2_mul(dx, dx), f2_mul(dy, dy)), f2_mul(dz, dz)), da, db);
-        da = __fsqrt_rn(da);
-        db = __fsqrt_rn(db);
-    } else {
-        f2_unpack(f2_add(f2_add(f2_mul(dx, f2_pack(a.w, a.w)), f2_mul(dy, f2_pack(b.x, b.x))), f2_mul(dz, f2_pack(b.y, b.y))),
-                  da, db);
-        da = fabsf(da);
-        db = fabsf(db);
-    }
-}
-
-// One window row of staged taps [row, row + 10) for up to two windows that
-// contain it (a vertical pixel pair's windows share nine of their rows): a
-// half row's taps are loaded once, before their comparisons, and each tap's
-// distances to both source points are evaluated together (packed pairs pa, pb
-// of the two points' coordinates: x, y, z).
-template <int kType>
-__device__ __forceinline__ void icp_scan_row(const float4 *sA, const float2 *sB, int row, f32x2 px, f32x2 py,
+// One window row of staged point-to-plane taps [row, row + 10) (column
+// quotients u, the row's quotient v) for up to two windows that contain it (a
+// vertical pixel pair's windows share nine of their rows): a half row's taps
+// are loaded once, before their comparisons, and each tap's distances
+// (kokkosICP.cpp:101-102) to both source points are evaluated together
+// (packed pairs of the two points' coordinates px, py, pz), with the
+// reference's roundings in its order.
+__device__ __forceinline__ void icp_scan_row(const float4 *sA, const float *u, float v, int row, f32x2 px, f32x2 py,
                                              f32x2 pz, bool ua, IcpBest &ba, bool ub, IcpBest &bb) {
 #pragma unroll
     for (int half = 0; half < 2; half++) {
         float4 a[kIcpSearch];
-        float2 b[kIcpSearch];
 #pragma unroll
-        for (int dl = 0; dl < kIcpSearch; dl++) {
-            a[dl] = sA[row + half * kIcpSearch + dl];
-            b[dl] = kType == SS_ICP_POINT_TO_PLANE ? sB[row + half * kIcpSearch + dl] : make_float2(0.f, 0.f);
-        }
+        for (int dl = 0; dl < kIcpSearch; dl++) a[dl] = sA[row + half * kIcpSearch + dl];
 #pragma unroll
         for (int dl = 0; dl < kIcpSearch; dl++) {
             const bool odd = ((dl + half * kIcpSearch) & 1) != 0;
             const int idx = row + half * kIcpSearch + dl;
+            const F3 y = icp_tap_point(a[dl], u[half * kIcpSearch + dl], v);
+            const f32x2 dx = f2_sub(f2_pack(y.x, y.x), px), dy = f2_sub(f2_pack(y.y, y.y), py),
+                        dz = f2_sub(f2_pack(y.z, y.z), pz);
             float da, db;
-            icp_tap_dist2<kType>(a[dl], b[dl], px, py, pz, da, db);
-            if (ua) ba.take(odd, da, idx);
-            if (ub) bb.take(odd, db, idx);
+            f2_unpack(f2_add(f2_add(f2_mul(dx, f2_pack(a[dl].y, a[dl].y)), f2_mul(dy, f2_pack(a[dl].z, a[dl].z))),
+                             f2_mul(dz, f2_pack(a[dl].w, a[dl].w))),
+                      da, db);
+            if (ua) ba.take(odd, fabsf(da), idx);
+            if (ub) bb.take(odd, fabsf(db), idx);
         }
     }
+}
+
+// The whole warp scans the point-to-plane windows of the lanes in todo, one
+// after the other, four taps a lane (base: the lane's window's first staged
+// row and column li, lj; pitch sw): the first tap of the reference's scan with
+// the smallest distance, as icp_scan_row's compare chains find it. Returns the
+// lane's tap (staged index) if it is in todo, else keep.
+__device__ __forceinline__ int icp_coop_plane(const float4 *sA, const float *su, unsigned todo, int li, int lj, int sw,
+                                              F3 px, int keep) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const F3 p{__shfl_sync(FULL, px.x, src), __shfl_sync(FULL, px.y, src), __shfl_sync(FULL, px.z, src)};
+        const int r0 = __shfl_sync(FULL, li, src), c0 = __shfl_sync(FULL, lj, src);
+        float smallest = kIcpMaxDist;
+        int tap = INT_MAX;
+#pragma unroll
+        for (int k = 0; k < 128; k += 32) {
+            const int t = k + lane;
+            if (t < 4 * kIcpSearch * kIcpSearch) {
+                const int r = r0 + t / (2 * kIcpSearch), c = c0 + t % (2 * kIcpSearch);
+                const float4 a = sA[r * sw + c];
+                const F3 y = icp_tap_point(a, su[c], su[kIcpEdge + r]);
+                const float dist = fabsf(f3dot(f3sub(y, p), F3{a.y, a.z, a.w}));
+                if (dist < smallest) {
+                    smallest = dist;
+                    tap = t;
+                }
+            }
+        }
+        const unsigned u = __float_as_uint(smallest), w = __reduce_min_sync(FULL, u);
+        const int t = (int)__reduce_min_sync(FULL, u == w ? (unsigned)tap : (unsigned)INT_MAX);
+        if (lane == src)
+            keep = t == INT_MAX ? -1 : (r0 + t / (2 * kIcpSearch)) * sw + c0 + t % (2 * kIcpSearch);
+    }
+    return keep;
+}
+
+// The nearest tap of a point-to-point window. The reference keeps the first
+// tap of its scan with the smallest rounded distance below max_dist
+// (kokkosICP.cpp:89-97). Two facts make 16 of the 100 taps enough for most
+// pixels:
+// - every tap of a column and row at least r pixels from the projected point
+//   lies on a viewing ray that passes the point at r |z| / (f |ray|) or more,
+//   so once the smallest distance found is below that (less 1 % for the
+//   roundings), no tap outside can be nearer. The window is taken in three
+//   squares around the centre: rows and columns -1..2 (16 taps; all others are
+//   2 pixels away or more), -2..3 (20 more; 3 pixels), -5..4 (the rest).
+//   Measured on noisy rooms a few pixels of a warp need more than the first;
+//   when they are few the whole warp takes one pixel at a time, a tap per lane.
+// - distances compare as their squares except where the square roots round to
+//   the same float. The two smallest squares are kept: where they lie within
+//   2^-21 of each other (a square root's rounding merges at most 2^-22), the
+//   window is scanned again with the rounded distances, in the reference's
+//   order.
+// With all 100 distances and their square roots evaluated a CTA's search took
+// 33 us on average at 640 x 480 (51 us until the last one, 27 at 160 x 120);
+// now 4 us (11-15 until the last one, 2 at 160 x 120).
+struct IcpNear {
+    float m1 = INFINITY, m2 = INFINITY;  // the two smallest squares
+    int b = -1;                          // the smallest's tap
+    __device__ __forceinline__ void take(float d2, int idx) {
+        b = d2 < m1 ? idx : b;
+        m2 = fminf(m2, fmaxf(m1, d2));
+        m1 = fminf(m1, d2);
+    }
+};
+constexpr float kIcpMaxD2 = kIcpMaxDist * kIcpMaxDist * 1.0001f;  // above the square of any accepted distance
+
+__device__ __forceinline__ float icp_dist2(const float4 a, F3 px) {
+    const F3 d = f3sub(F3{a.x, a.y, a.z}, px);
+    return f3dot(d, d);
+}
+
+// Tap t of the second square without the first (20), and of the window
+// without the second square (64), as row and column offsets from the centre.
+__device__ __forceinline__ void icp_ring(int t, int &dk, int &dl) {
+    if (t < 12) {
+        dk = t < 6 ? -2 : 3;
+        dl = (t < 6 ? t : t - 6) - 2;
+    } else {
+        dk = ((t - 12) & 3) - 1;
+        dl = t < 16 ? -2 : 3;
+    }
+}
+__device__ __forceinline__ void icp_rim(int t, int &dk, int &dl) {
+    if (t < 40) {
+        const int r = t / 10;
+        dk = r < 3 ? r - 5 : 4;
+        dl = t - 10 * r - 5;
+    } else {
+        const int c = t & 3;
+        dk = ((t - 40) >> 2) - 2;
+        dl = c < 3 ? c - 5 : 4;
+    }
+}
+
+// The warp's smallest and second smallest of the lanes' states (non-negative
+// squares, compared as integers), into lane src's state.
+__device__ __forceinline__ void icp_merge(IcpNear &s, IcpNear mine, int src) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned u1 = __float_as_uint(mine.m1);
+    const unsigned w1 = __reduce_min_sync(FULL, u1);
+    const int who = __ffs(__ballot_sync(FULL, u1 == w1)) - 1;
+    const unsigned w2 = __reduce_min_sync(FULL, lane == who ? __float_as_uint(mine.m2) : u1);
+    const int b = __shfl_sync(FULL, mine.b, who);
+    if (lane == src) {
+        const float f1 = __uint_as_float(w1), f2 = __uint_as_float(w2);
+        s.b = f1 < s.m1 ? b : s.b;
+        s.m2 = fminf(fminf(s.m2, f2), fmaxf(s.m1, f1));
+        s.m1 = fminf(s.m1, f1);
+    }
+}
+
+// The staged index of the correspondence of a source point px (valid: the
+// reference searches), or -1; base: the centre's staged index, sw the row
+// pitch. Every lane of the warp calls it.
+__device__ __forceinline__ int icp_search_point(const float4 *sA, bool valid, int base, int sw, F3 px, Intr in) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    IcpNear s;
+    if (valid) {
+#pragma unroll
+        for (int dk = -1; dk <= 2; dk++)
+#pragma unroll
+            for (int dl = -1; dl <= 2; dl++) {
+                const int t = base + dk * sw + dl;
+                s.take(icp_dist2(sA[t], px), t);
+            }
+    }
+    // q r^2: the least square of a tap r pixels away; the window's rays have
+    // |x| <= |px.x| + 6 |z| / fx at depth z, and y likewise
+    const float ax = 1.f / fabsf(in.fx), ay = 1.f / fabsf(in.fy), z = fabsf(px.z), am = fminf(ax, ay);
+    const float wx = fmaf(6.f * ax, z, fabsf(px.x)), wy = fmaf(6.f * ay, z, fabsf(px.y)), z2 = z * z;
+    const float q = 0.99f * (am * am) * (z2 * z2) / fmaf(wx, wx, fmaf(wy, wy, z2));
+    const bool more = valid && !(fminf(s.m1, kIcpMaxD2) < 4.f * q);
+    unsigned todo = __ballot_sync(FULL, more);
+    if (__popc(todo) > kIcpCoop) {
+        if (more) {
+#pragma unroll 4
+            for (int t = 0; t < 20; t++) {
+                int dk, dl;
+                icp_ring(t, dk, dl);
+                const int i = base + dk * sw + dl;
+                s.take(icp_dist2(sA[i], px), i);
+            }
+            if (!(fminf(s.m1, kIcpMaxD2) < 9.f * q)) {
+#pragma unroll 4
+                for (int t = 0; t < 64; t++) {
+                    int dk, dl;
+                    icp_rim(t, dk, dl);
+                    const int i = base + dk * sw + dl;
+                    s.take(icp_dist2(sA[i], px), i);
+                }
+            }
+        }
+    } else {
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const F3 p{__shfl_sync(FULL, px.x, src), __shfl_sync(FULL, px.y, src), __shfl_sync(FULL, px.z, src)};
+            const int c = __shfl_sync(FULL, base, src);
+            IcpNear mine;
+            int dk, dl;
+            if (lane < 20) {
+                icp_ring(lane, dk, dl);
+                const int i = c + dk * sw + dl;
+                mine.take(icp_dist2(sA[i], p), i);
+            }
+            icp_merge(s, mine, src);
+            if (__shfl_sync(FULL, fminf(s.m1, kIcpMaxD2) < 9.f * q ? 1 : 0, src)) continue;
+            mine = IcpNear{};
+#pragma unroll
+            for (int t = 0; t < 64; t += 32) {
+                icp_rim(t + lane, dk, dl);
+                const int i = c + dk * sw + dl;
+                mine.take(icp_dist2(sA[i], p), i);
+            }
+            icp_merge(s, mine, src);
+        }
+    }
+    if (!(s.m1 <= kIcpMaxD2)) return -1;
+    if (s.m2 <= __fmul_ru(s.m1, 1.0000005f)) {  // square roots that may round alike: the reference's scan
+        float smallest = kIcpMaxDist;
+        int b = -1;
+        for (int dk = -kIcpSearch; dk < kIcpSearch; dk++)
+            for (int dl = -kIcpSearch; dl < kIcpSearch; dl++) {
+                const int i = base + dk * sw + dl;
+                const float dist = __fsqrt_rn(icp_dist2(sA[i], px));
+                if (dist < smallest) {
+                    smallest = dist;
+                    b = i;
+                }
+            }
+        return b;
+    }
+    return __fsqrt_rn(s.m1) < kIcpMaxDist ? s.b : -1;
 }
 
 // A window read from global memory (a tile whose window region does not fit
 // the stage): image indices, the reference's loops.
 template <int kType>
-__device__ __forceinline__ int icp_search_global(const float4 *__restrict__ ya, const float2 *__restrict__ yb, int cols,
+__device__ __forceinline__ int icp_search_global(const float4 *__restrict__ ya, const float *__restrict__ uv, int cols,
                                                  int ci, int cj, F3 px) {
-    IcpBest bt;
-    for (int k = ci - kIcpSearch; k < ci + kIcpSearch; k++)
+    float smallest = kIcpMaxDist;
+    int b = -1;
+    for (int k = ci - kIcpSearch; k < ci + kIcpSearch; k++) {
+        const float v = __ldg(uv + cols + k);
         for (int l = cj - kIcpSearch; l < cj + kIcpSearch; l++) {
             const int tag = k * cols + l;
-            const float2 b = kType == SS_ICP_POINT_TO_PLANE ? __ldg(yb + tag) : make_float2(0.f, 0.f);
-            bt.take(false, icp_tap_dist<kType>(__ldg(ya + tag), b, px), tag);
+            const float4 a = __ldg(ya + tag);
+            const float dist =
+                kType == SS_ICP_POINT_TO_POINT
+                    ? __fsqrt_rn(icp_dist2(a, px))
+                    : fabsf(f3dot(f3sub(icp_tap_point(a, __ldg(uv + l), v), px), F3{a.y, a.z, a.w}));
+            if (dist < smallest) {
+                smallest = dist;
+                b = tag;
+            }
         }
-    return bt.best();
+    }
+    return b;
 }
 
-// Adds one source pixel's terms of the host sums (kokkosICP.cpp:121-171) to
-// the lane's float pairs: for a correspondence (x_nearest.z != 0) the count,
-// x, x_nearest, x x_nearest^T (each product exact as a pair) and the RMSE
-// term. best indexes the staged region (staged) or the image.
+// One source pixel's terms of the host sums (kokkosICP.cpp:121-171) as float
+// pairs: x, x_nearest, x x_nearest^T (each product exact as a pair) and the
+// RMSE term; false (and zeros) without a correspondence (x_nearest.z == 0,
+// :131). a: the best tap's entry, y its point (point to plane).
 template <int kType>
-__device__ __forceinline__ void icp_add_terms(F3 x, const Mat34 &T, int best, bool staged, const float4 *sA,
-                                              const float2 *sB, const float4 *__restrict__ ya,
-                                              const float2 *__restrict__ yb, float *vh, float *vl) {
-    if (best < 0) return;
-    const F3 px = xform(T, x);
-    const float4 a = staged ? sA[best] : __ldg(ya + best);
-    const float2 b = kType == SS_ICP_POINT_TO_PLANE ? (staged ? sB[best] : __ldg(yb + best)) : make_float2(0.f, 0.f);
-    const F3 py{a.x, a.y, a.z}, nn{a.w, b.x, b.y};
-    const F3 bpt = kType == SS_ICP_POINT_TO_POINT ? py : f3add(px, f3smul(f3dot(f3sub(py, px), nn), nn));
-    if (bpt.z == 0) return;  // x_nearest(i, j).z == 0: no correspondence (kokkosICP.cpp:131)
-    const float xa[3] = {x.x, x.y, x.z}, xb[3] = {bpt.x, bpt.y, bpt.z};
-    fp2_add(vh[0], vl[0], 1.f, 0.f);
+__device__ __forceinline__ bool icp_terms(F3 x, const Mat34 &T, bool found, float4 a, F3 y, float *vh, float *vl) {
+    F3 b{0.f, 0.f, 0.f};
+    if (found) {
+        if (kType == SS_ICP_POINT_TO_POINT) {
+            b = F3{a.x, a.y, a.z};
+        } else {
+            const F3 px = xform(T, x), nn{a.y, a.z, a.w};
+            b = f3add(px, f3smul(f3dot(f3sub(y, px), nn), nn));
+        }
+    }
+    const bool ok = b.z != 0;
+    const float xa[3] = {ok ? x.x : 0.f, ok ? x.y : 0.f, ok ? x.z : 0.f}, xb[3] = {b.x, b.y, b.z};
 #pragma unroll
     for (int r = 0; r < 3; r++) {
-        fp2_add(vh[1 + r], vl[1 + r], xa[r], 0.f);
-        fp2_add(vh[4 + r], vl[4 + r], xb[r], 0.f);
+        vh[r] = xa[r];
+        vl[r] = 0.f;
+        vh[3 + r] = ok ? xb[r] : 0.f;
+        vl[3 + r] = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; c++) {  // x y^T, each product exact as a pair
             const float q = __fmul_rn(xa[r], xb[c]);
-            fp2_add(vh[7 + 3 * r + c], vl[7 + 3 * r + c], q, fmaf(xa[r], xb[c], -q));
+            vh[6 + 3 * r + c] = q;
+            vl[6 + 3 * r + c] = fmaf(xa[r], xb[c], -q);
         }
     }
     // RMSE term || x_nearest - Txy x || squared in float (kokkosICP.cpp:137-138; the
@@ -608,24 +824,32 @@ __device__ __forceinline__ void icp_add_terms(F3 x, const Mat34 &T, int best, bo
     const float e1 = xb[1] - fmaf(T.m[4], xa[0], fmaf(T.m[5], xa[1], fmaf(T.m[6], xa[2], T.m[7])));
     const float e2 = xb[2] - fmaf(T.m[8], xa[0], fmaf(T.m[9], xa[1], fmaf(T.m[10], xa[2], T.m[11])));
     const float tmp = sqrtf(fmaf(e0, e0, fmaf(e1, e1, e2 * e2)));
-    fp2_add(vh[16], vl[16], tmp * tmp, 0.f);
+    vh[15] = ok ? tmp * tmp : 0.f;
+    vl[15] = 0.f;
+    return ok;
 }
 
 // Copies the target entries of rows [r0, r0 + h) x columns [q0, q0 + w) of
 // the image into the stage (row pitch w) with asynchronous copies: warp k
 // copies rows k, k + 8, ..., its lanes the columns, the entries in the layout
-// icp_prep_kernel wrote them in. The caller waits for them.
+// icp_prep_kernel wrote them in; point to plane with their columns' and rows'
+// quotients (su: columns, then from kIcpEdge rows). The caller waits for them.
 template <int kType>
-__device__ __forceinline__ void icp_stage(float4 *sA, float2 *sB, const float4 *__restrict__ ya,
-                                          const float2 *__restrict__ yb, int cols, int r0, int q0, int w, int h) {
-    const unsigned sa_s = (unsigned)__cvta_generic_to_shared(sA), sb_s = (unsigned)__cvta_generic_to_shared(sB);
+__device__ __forceinline__ void icp_stage(float4 *sA, float *su, const float4 *__restrict__ ya,
+                                          const float *__restrict__ uv, int cols, int r0, int q0, int w, int h) {
+    const unsigned sa_s = (unsigned)__cvta_generic_to_shared(sA);
+    if (kType == SS_ICP_POINT_TO_PLANE) {
+        const unsigned su_s = (unsigned)__cvta_generic_to_shared(su);
+        const int t = threadIdx.x;  // w, h <= kIcpEdge < 256
+        if (t < w) cp_async4(su_s + 4u * t, uv + q0 + t);
+        if (t < h) cp_async4(su_s + 4u * (kIcpEdge + t), uv + cols + r0 + t);
+    }
     const int ln = threadIdx.x & 31;
     for (int r = threadIdx.x >> 5; r < h; r += 8) {
         const size_t q = (size_t)(r0 + r) * cols + q0;
         for (int c = ln; c < w; c += 32) {
             const int t = r * w + c;
             cp_async16(sa_s + 16u * t, ya + q + c);
-            if (kType == SS_ICP_POINT_TO_PLANE) cp_async8(sb_s + 8u * t, yb + q + c);
         }
     }
 }
@@ -640,8 +864,8 @@ constexpr int kIcpMargin = 2;
 // vertical pair (rows 2w and 2w + 1 of warp w's lane column). The target
 // points and normals under the tile's windows are staged in shared memory
 // first by asynchronous copies of icp_prep_kernel's entries (a tap that the
-// reference skips holding NaN, so that its distance fails every comparison).
-// The search keeps the reference's scan order and strict comparisons for
+// reference skips holding NaN or infinity, so that its distance fails every
+// comparison). The point-to-plane search keeps the reference's scan order and strict comparisons for
 // each window, remembers the best tap and forms the correspondence from it
 // afterwards. Every iteration after the first stages, before it waits for
 // the previous one, the region its CTA needed there widened by kIcpMargin
@@ -651,17 +875,23 @@ constexpr int kIcpMargin = 2;
 // only its bounds matter. When the two windows lie in the same columns at most two rows
 // apart (the usual case: neighbouring pixels project to neighbouring centres,
 // one row apart), the thread scans their union, loading each tap once for
-// both; otherwise it scans the lower window on its own after the upper one.
+// both; the few lower windows that do not join are left to the whole warp
+// (icp_coop_plane: one lane's scan of its own cost its warp as much as the
+// joined one, and most warps held one: 24 -> 18 us until the last CTA's
+// search ends at 640 x 480). A point-to-plane tap is one 16-byte entry, its
+// point rebuilt from its depth and the staged quotients (24-byte entries kept
+// the shared-memory pipe busiest; now it is the FP32 pipe, two products more
+// a tap). Point to point: icp_search_point, pixel by pixel.
 // 64 registers (four CTAs per SM; only the rank-deficient fallback of the
 // last CTA spills).
 template <int kType>
 __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__restrict__ xp,
                                                            const float4 *__restrict__ ya,
-                                                           const float2 *__restrict__ yb, int rows, int cols, Intr in,
+                                                           const float *__restrict__ uv, int rows, int cols, Intr in,
                                                            IcpState *st,
                                                            int4 *__restrict__ regions, int prestage, IcpOut *out) {
-    __shared__ float4 sA[kIcpStage];  // target (x, y, z, nx)
-    __shared__ float2 sB[kIcpStage];  // target (ny, nz)
+    __shared__ float4 sA[kIcpStage];      // target entries
+    __shared__ float su[2 * kIcpEdge];    // point to plane: the staged columns' and rows' quotients
     __shared__ float2 red[8][kIcpSums];
     __shared__ int box[4];
     __shared__ int4 pre;
@@ -681,7 +911,7 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
             // read only costs the restaging: it is checked to lie in the image)
             const int4 R = __ldcg(regions + cta);
             int4 q = make_int4(0, 0, 0, 0);
-            if (R.z > 0 && R.w > 0 && R.x >= 0 && R.y >= 0 && R.w <= rows - R.x && R.z <= cols - R.y)
+            if (R.z > 0 && R.w > 0 && R.z <= kIcpEdge - 2 * kIcpMargin && R.w <= kIcpEdge - 2 * kIcpMargin && R.x >= 0 && R.y >= 0 && R.w <= rows - R.x && R.z <= cols - R.y)
                 for (int m = kIcpMargin; m >= 0; m--) {
                     const int a0 = max(R.x - m, 0), b0 = max(R.y - m, 0);
                     const int a1 = min(R.x + R.w + m, rows), b1 = min(R.y + R.z + m, cols);
@@ -694,7 +924,7 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
         }
         __syncthreads();
         P = pre;
-        if (P.w > 0) icp_stage<kType>(sA, sB, ya, yb, cols, P.x, P.y, P.z, P.w);
+        if (P.w > 0) icp_stage<kType>(sA, su, ya, uv, cols, P.x, P.y, P.z, P.w);
     }
     pdl_wait();
     Mat34 T;
@@ -748,14 +978,18 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
             __syncthreads();
         }
         // inside the image: the border test keeps every window within rows x cols
-        icp_stage<kType>(sA, sB, ya, yb, cols, r0, q0, W, H);
+        icp_stage<kType>(sA, su, ya, uv, cols, r0, q0, W, H);
     }
     cp_async_wait_all();
     if (threadIdx.x == 0) regions[cta] = any ? make_int4(r0, q0, W, H) : make_int4(0, 0, 0, 0);
     __syncthreads();
 
     int best0 = -1, best1 = -1;
-    if (staged) {
+    if (staged && kType == SS_ICP_POINT_TO_POINT) {
+        const int o = sr0 * sw + sq0;
+        best0 = icp_search_point(sA, sa, ca_i * sw + ca_j - o, sw, pa, in);
+        best1 = icp_search_point(sA, sb, cb_i * sw + cb_j - o, sw, pb, in);
+    } else if (staged) {
         // the thread's windows: the upper one leads, and the other joins it
         // when it lies dr = 0..2 rows below in the same columns (its rows are
         // then the lead's rows dr..dr + 9); a lower window that does not join
@@ -771,36 +1005,75 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
         const f32x2 qx = f2_pack(pl.x, pm.x), qy = f2_pack(pl.y, pm.y), qz = f2_pack(pl.z, pm.z);
         IcpBest bl, bm;
         if (sa || sb) {
-            const int li = swap ? cb_i : ca_i, lj = swap ? cb_j : ca_j;
-            const int base = (li - kIcpSearch - sr0) * sw + (lj - kIcpSearch - sq0);
+            const int li = (swap ? cb_i : ca_i) - kIcpSearch - sr0, lj = (swap ? cb_j : ca_j) - kIcpSearch - sq0;
+            float u[2 * kIcpSearch];
+#pragma unroll
+            for (int k = 0; k < 2 * kIcpSearch; k++) u[k] = su[lj + k];
             const int nr = 2 * kIcpSearch + dr;
 #pragma unroll 1
             for (int dk = 0; dk < nr; dk++)
-                icp_scan_row<kType>(sA, sB, base + dk * sw, qx, qy, qz, dk < 2 * kIcpSearch, bl, joined && dk >= dr, bm);
+                icp_scan_row(sA, u, su[kIcpEdge + li + dk], (li + dk) * sw + lj, qx, qy, qz, dk < 2 * kIcpSearch, bl,
+                             joined && dk >= dr, bm);
         }
-        if (sa && sb && !joined) {  // the lower window on its own (the upper one led)
-            const int base = (cb_i - kIcpSearch - sr0) * sw + (cb_j - kIcpSearch - sq0);
-            const f32x2 ux = f2_pack(pb.x, pb.x), uy = f2_pack(pb.y, pb.y), uz = f2_pack(pb.z, pb.z);
+        // the lower windows that did not join (the upper one led): a few of a
+        // warp's are scanned by the whole warp (one lane's own scan would cost
+        // the warp as much as all lanes'), many by their lanes
+        int tail = -1;
+        const bool rest = sa && sb && !joined;
+        const unsigned todo = __ballot_sync(0xffffffffu, rest);
+        if (todo) {
+            const int li = cb_i - kIcpSearch - sr0, lj = cb_j - kIcpSearch - sq0;
+            if (__popc(todo) <= kIcpCoop) {
+                tail = icp_coop_plane(sA, su, todo, li, lj, sw, pb, -1);
+            } else if (rest) {
+                float u[2 * kIcpSearch];
+#pragma unroll
+                for (int k = 0; k < 2 * kIcpSearch; k++) u[k] = su[lj + k];
+                const f32x2 ux = f2_pack(pb.x, pb.x), uy = f2_pack(pb.y, pb.y), uz = f2_pack(pb.z, pb.z);
 #pragma unroll 1
-            for (int dk = 0; dk < 2 * kIcpSearch; dk++)
-                icp_scan_row<kType>(sA, sB, base + dk * sw, ux, uy, uz, true, bm, false, bl);
+                for (int dk = 0; dk < 2 * kIcpSearch; dk++)
+                    icp_scan_row(sA, u, su[kIcpEdge + li + dk], (li + dk) * sw + lj, ux, uy, uz, true, bm, false, bl);
+                tail = bm.best();
+            }
         }
         best0 = swap ? bm.best() : bl.best();
-        best1 = swap ? bl.best() : bm.best();
+        best1 = rest ? tail : swap ? bl.best() : bm.best();
     } else {
-        if (sa) best0 = icp_search_global<kType>(ya, yb, cols, ca_i, ca_j, pa);
-        if (sb) best1 = icp_search_global<kType>(ya, yb, cols, cb_i, cb_j, pb);
+        if (sa) best0 = icp_search_global<kType>(ya, uv, cols, ca_i, ca_j, pa);
+        if (sb) best1 = icp_search_global<kType>(ya, uv, cols, cb_i, cb_j, pb);
     }
 
-    // this thread's terms as float pairs, padded to 32 for the transpose-reduce
-    float vh[32], vl[32];
+    // this thread's terms as float pairs (values 1..16) and the warp's counts
+    auto entry = [&](int best, F3 &y) {
+        y = F3{0.f, 0.f, 0.f};
+        if (best < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 a = staged ? sA[best] : __ldg(ya + best);
+        if (kType == SS_ICP_POINT_TO_PLANE) {
+            const int pitch = staged ? sw : cols, r = (int)((unsigned)best / (unsigned)pitch), c = best - r * pitch;
+            y = icp_tap_point(a, staged ? su[c] : __ldg(uv + c), staged ? su[kIcpEdge + r] : __ldg(uv + cols + r));
+        }
+        return a;
+    };
+    float vh[kIcpPairs], vl[kIcpPairs];
+    F3 y0, y1;
+    const float4 a0 = entry(best0, y0), a1 = entry(best1, y1);
+    const bool ok0 = icp_terms<kType>(x0, T, best0 >= 0, a0, y0, vh, vl);
+    bool ok1;
+    {
+        float wh[kIcpPairs], wl[kIcpPairs];
+        ok1 = icp_terms<kType>(x1, T, best1 >= 0, a1, y1, wh, wl);
 #pragma unroll
-    for (int k = 0; k < 32; k++) vh[k] = vl[k] = 0.f;
-    vh[17] = (float)((x0.z != 0) + (x1.z != 0));  // n_pointsinX
-    icp_add_terms<kType>(x0, T, best0, staged, sA, sB, ya, yb, vh, vl);
-    icp_add_terms<kType>(x1, T, best1, staged, sA, sB, ya, yb, vh, vl);
+        for (int k = 0; k < kIcpPairs; k += 2) {
+            f32x2 h = f2_pack(vh[k], vh[k + 1]), l = f2_pack(vl[k], vl[k + 1]);
+            fp2_add2(h, l, f2_pack(wh[k], wh[k + 1]), f2_pack(wl[k], wl[k + 1]));
+            f2_unpack(h, vh[k], vh[k + 1]);
+            f2_unpack(l, vl[k], vl[k + 1]);
+        }
+    }
     const int lane = threadIdx.x & 31;
-    const float2 csum = icp_cta_sum(vh, vl, red);
+    const int n_cors = __popc(__ballot_sync(0xffffffffu, ok0)) + __popc(__ballot_sync(0xffffffffu, ok1));
+    const int n_x = __popc(__ballot_sync(0xffffffffu, x0.z != 0)) + __popc(__ballot_sync(0xffffffffu, x1.z != 0));
+    const float2 csum = icp_cta_sum(vh, vl, n_cors, n_x, red);
     // the CTA's sums into the fixed-point words (thread v < kIcpSums: value v)
     if (threadIdx.x < kIcpSums) {
         __int128 qh, ql;
@@ -946,33 +1219,41 @@ static inline int icp_tiles_y(int rows) { return (rows + 15) / 16; }
 struct IcpWorkspace {
     float *xp = nullptr;
     float4 *ya = nullptr;
-    float2 *yb = nullptr;
+    float *uv = nullptr;  // the target's column and row quotients
     int4 *regions = nullptr;
     IcpState *state = nullptr;
     IcpOut *out_host = nullptr, *out_dev = nullptr;  // pinned, mapped
     size_t npix = 0;
+    int sides = 0;  // rows + cols
     int ctas = 0;
 };
 static std::mutex g_icp_mutex;
 static IcpWorkspace g_icp_ws[64];
 
-static ss_status icp_workspace(int dev, size_t npix, int ctas, IcpWorkspace **out) {
+static ss_status icp_workspace(int dev, size_t npix, int sides, int ctas, IcpWorkspace **out) {
     if (dev < 0 || dev >= 64) return SS_ERR_ARG;
     IcpWorkspace &w = g_icp_ws[dev];
     if (w.npix < npix) {
         cudaFree(w.xp);
         cudaFree(w.ya);
-        cudaFree(w.yb);
         w.xp = nullptr;
         w.ya = nullptr;
-        w.yb = nullptr;
         w.npix = 0;
-        if (cudaMalloc(&w.xp, npix * 12) != cudaSuccess || cudaMalloc(&w.ya, npix * 16) != cudaSuccess ||
-            cudaMalloc(&w.yb, npix * 8) != cudaSuccess) {
+        if (cudaMalloc(&w.xp, npix * 12) != cudaSuccess || cudaMalloc(&w.ya, npix * 16) != cudaSuccess) {
             cudaGetLastError();
             return SS_ERR_NOMEM;
         }
         w.npix = npix;
+    }
+    if (w.sides < sides) {
+        cudaFree(w.uv);
+        w.uv = nullptr;
+        w.sides = 0;
+        if (cudaMalloc(&w.uv, (size_t)sides * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            return SS_ERR_NOMEM;
+        }
+        w.sides = sides;
     }
     if (w.ctas < ctas || !w.state) {
         cudaFree(w.regions);
@@ -1054,7 +1335,7 @@ static void orthonormalize_rotation(double *T) {
 // it there and the call ends with a stream synchronisation; without, the
 // state is copied back.
 ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols, Intr in, const double tx[16],
-                      const double ty[16], int type, float *xp, float4 *ya, float2 *yb, int ctas,
+                      const double ty[16], int type, float *xp, float4 *ya, float *uv, int ctas,
                       int4 *regions, IcpState *state, IcpOut *out_host, IcpOut *out_dev, double txy_out[16],
                       float *rmse_out, cudaStream_t s) {
     // Txy = ty^-1 * tx (kokkosICP.cpp:57), float copy for the search
@@ -1069,7 +1350,7 @@ ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols
     IcpInit ini;
     for (int k = 0; k < 16; k++) ini.Txy[k] = (float)T[k];
     const dim3 blk(128), grid((cols + 127) / 128, rows);
-    icp_prep_kernel<<<grid, blk, 0, s>>>(d1, d2, rows, cols, in, type, xp, ya, yb, ini, state);
+    icp_prep_kernel<<<grid, blk, 0, s>>>(d1, d2, rows, cols, in, type, xp, ya, uv, ini, state);
     SS_LAUNCH_CHECK();
     const dim3 tiles(icp_tiles_x(cols), icp_tiles_y(rows));  // ctas == tiles.x * tiles.y
     // four CTAs per SM (64 registers, 38 KB of shared memory each) need the
@@ -1088,10 +1369,10 @@ ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols
         IcpOut *o = it == kIcpIters - 1 ? out_dev : nullptr;
         if (type == SS_ICP_POINT_TO_POINT)
             SS_CUDA_TRY(launch_kernel(icp_ref_iter_kernel<SS_ICP_POINT_TO_POINT>, tiles, dim3(256), 0, s, it > 0, xp, ya,
-                                      yb, rows, cols, in, state, regions, (int)(it > 0), o));
+                                      uv, rows, cols, in, state, regions, (int)(it > 0), o));
         else
             SS_CUDA_TRY(launch_kernel(icp_ref_iter_kernel<SS_ICP_POINT_TO_PLANE>, tiles, dim3(256), 0, s, it > 0, xp, ya,
-                                      yb, rows, cols, in, state, regions, (int)(it > 0), o));
+                                      uv, rows, cols, in, state, regions, (int)(it > 0), o));
     }
     float2 best[16];
     float lowest;
@@ -1132,9 +1413,9 @@ constexpr size_t kNoAllocMaxPixels = 640 * 480;  // largest rows * cols accepted
 constexpr int kNoAllocCtas = 4096;  // iteration-grid CTAs (32 x 16 tiles): any rows x cols <= 640 x 480 needs <= 1600
 constexpr size_t kAlign256(size_t n) { return (n + 255) / 256 * 256; }
 constexpr size_t kNoAllocSource = kAlign256(kNoAllocMaxPixels * 12);  // source points
-constexpr size_t kNoAllocTargetA = kAlign256(kNoAllocMaxPixels * 16);  // target (x, y, z, nx)
-constexpr size_t kNoAllocTargetB = kAlign256(kNoAllocMaxPixels * 8);   // target (ny, nz)
-constexpr size_t kNoAllocImages = kNoAllocSource + kNoAllocTargetA + kNoAllocTargetB;
+constexpr size_t kNoAllocTarget = kAlign256(kNoAllocMaxPixels * 16);  // target entries
+constexpr size_t kNoAllocSides = kAlign256(kNoAllocMaxPixels * 4);    // column and row quotients (rows + cols <= rows * cols)
+constexpr size_t kNoAllocImages = kNoAllocSource + kNoAllocTarget + kNoAllocSides;
 constexpr size_t kNoAllocRegions = kAlign256((size_t)kNoAllocCtas * sizeof(int4));  // staged region per CTA
 constexpr size_t kNoAllocBytes = kNoAllocImages + kNoAllocRegions + kAlign256(sizeof(IcpState));
 
@@ -1252,11 +1533,11 @@ ss_status ss_kokkos_icp_noalloc(const uint16_t *d1, const uint16_t *d2, int32_t 
     if (st != SS_OK) return st;
     float *xp = (float *)base;
     float4 *ya = (float4 *)(base + kNoAllocSource);
-    float2 *yb = (float2 *)(base + kNoAllocSource + kNoAllocTargetA);
+    float *uv = (float *)(base + kNoAllocSource + kNoAllocTarget);
     int4 *regions = (int4 *)(base + kNoAllocImages);
     IcpState *state = (IcpState *)(base + kNoAllocImages + kNoAllocRegions);
     const Intr in{fx, fy, (float)rows - cy, cx};
-    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, xp, ya, yb, ctas, regions, state, nullptr,
+    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, xp, ya, uv, ctas, regions, state, nullptr,
                        nullptr, txy_out,
                        rmse_out, (cudaStream_t)stream);
 }
@@ -1288,10 +1569,10 @@ ss_status ss_kokkos_icp(const uint16_t *d1, const uint16_t *d2, int32_t rows, in
     const int ctas = icp_tiles_x(cols) * icp_tiles_y(rows);
     std::lock_guard<std::mutex> lock(g_icp_mutex);
     IcpWorkspace *w = nullptr;
-    st = icp_workspace(dev, (size_t)rows * cols, ctas, &w);
+    st = icp_workspace(dev, (size_t)rows * cols, rows + cols, ctas, &w);
     if (st != SS_OK) return st;
     const Intr in{fx, fy, (float)rows - cy, cx};  // ci = resi - cy, cj = cx (kokkosICP.cpp:48-49)
-    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, w->xp, w->ya, w->yb, ctas, w->regions,
+    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, w->xp, w->ya, w->uv, ctas, w->regions,
                        w->state, w->out_host, w->out_dev,
                        txy_out, rmse_out, (cudaStream_t)stream);
 }
