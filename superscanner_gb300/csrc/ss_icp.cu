@@ -364,15 +364,16 @@ __device__ bool polar3_warp_f32(const float *Hf, float *R) {
         // y is the reciprocal of the g det that scales X
         const float g = rsqrtf(rsqrtf(__fdividef(fc, det * det * fx)));
         const float y = __frcp_rn(g * det);
-        float dlt = 0.f;
+        float d[9];
 #pragma unroll
         for (int k = 0; k < 9; k++) {
             const float xn = 0.5f * fmaf(g, X[k], cof[k] * y);
-            dlt = fmaxf(dlt, fabsf(xn - X[k]));
+            d[k] = fabsf(xn - X[k]);
             X[k] = xn;
         }
         if (last) break;
-        last = dlt <= 1e-4f;
+        last = fmaxf(fmaxf(fmaxf(fmaxf(d[0], d[1]), fmaxf(d[2], d[3])), fmaxf(fmaxf(d[4], d[5]), fmaxf(d[6], d[7]))),
+                     d[8]) <= 1e-4f;
     }
     if (!last) return false;
     const int lane = threadIdx.x & 31;
@@ -1095,27 +1096,68 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
     __syncthreads();
     if (!last) return;  // (a CTA's exit lets the next iteration launch)
     pdl_trigger();      // the next iteration may launch (it waits for this grid before reading anything it writes)
-    if (threadIdx.x >= 32) return;
-    // last CTA, warp 0: lane v < kIcpSums takes total v as a float pair and
-    // clears its words for the next iteration
-    const float lowest = *(volatile float *)&st->lowest;  // the best RMSE so far
+    if (threadIdx.x >= 64) return;
+    // last CTA: lane v < kIcpSums of warps 0 and 1 takes total v as a float
+    // pair. Warp 0 forms the transform; warp 1 meanwhile the RMSE and the
+    // fitness, then (the words having been read) clears the words and writes
+    // the rest of the next iteration's state: after the transform on one warp
+    // these took 1000 cycles of the serial path
     __shared__ float2 tot[kIcpSums];
     __shared__ double Hs[9], Rs[9];
     __shared__ float Hf[9], Rf[9];
+    __shared__ int better;
+    __shared__ float low;
+    const bool side = threadIdx.x >= 32;
+    const int overflow = __ldcg(&st->overflow);
+    float2 v = make_float2(0.f, 0.f);
     if (lane < kIcpSums) {
-        unsigned long long *w = st->acc + 3 * lane;
+        const unsigned long long *w = st->acc + 3 * lane;
         const unsigned long long s0 = __ldcg(w), s1 = __ldcg(w + 1), s2 = __ldcg(w + 2);
-        w[0] = 0ull;
-        w[1] = 0ull;
-        w[2] = 0ull;
         const __int128 t = fixed48_total(s0, s1, s2);
         const float h = icp_float_of_fixed(t);
         __int128 hq;
         fixed48_of_float(h, hq);
-        float2 v = make_float2(h, icp_float_of_fixed(t - hq));
-        if (*(volatile int *)&st->overflow) v = make_float2(__int_as_float(0x7fc00000), 0.f);  // as the reference's NaNs
-        tot[lane] = v;
+        v = make_float2(h, icp_float_of_fixed(t - hq));
+        if (overflow) v = make_float2(__int_as_float(0x7fc00000), 0.f);  // as the reference's NaNs
     }
+    // named barriers between the two warps: 1, warp 0 has read the words; 2, better and low are set
+    if (!side) asm volatile("bar.arrive 1, 64;" ::: "memory");
+    if (side) {
+        const float lowest = __ldcg(&st->lowest), best_fitness = __ldcg(&st->best_fitness);  // so far
+        const int it = __ldcg(&st->iteration);
+        const float n = __shfl_sync(0xffffffffu, v.x, 0);
+        float rsme = __shfl_sync(0xffffffffu, v.x, 16);
+        rsme /= n;
+        rsme = sqrtf(rsme);
+        const float fitness = n / __shfl_sync(0xffffffffu, v.x, 17);
+        const bool became_best = rsme < lowest;  // kokkosICP.cpp:181-185
+        if (lane == 0) {
+            better = became_best;
+            low = became_best ? rsme : lowest;
+        }
+        asm volatile("bar.arrive 2, 64;" ::: "memory");
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        if (lane < kIcpSums) {
+            unsigned long long *w = st->acc + 3 * lane;
+            w[0] = 0ull;
+            w[1] = 0ull;
+            w[2] = 0ull;
+        }
+        if (lane != 0) return;
+        if (became_best) st->lowest = rsme;
+        if (fitness > best_fitness) st->best_fitness = fitness;
+        if (it < kIcpIters) {
+            st->stats[it * 4 + 0] = n;
+            st->stats[it * 4 + 1] = rsme;
+            st->stats[it * 4 + 2] = fitness;
+            st->stats[it * 4 + 3] = became_best ? 1.f : 0.f;
+        }
+        st->iteration = it + 1;
+        st->ticket = 0;
+        st->overflow = 0;
+        return;
+    }
+    if (lane < kIcpSums) tot[lane] = v;
     __syncwarp();
     // the update in float pairs (no FP64 instruction on this serial path; the
     // reference forms it in double, kokkosICP.cpp:121-185): n is an exact count
@@ -1186,29 +1228,13 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
         }
     }
     if (lane < 16) st->Txy[lane] = tn.x;
-    float rsme = tot[16].x;
-    rsme /= n;
-    rsme = sqrtf(rsme);
-    const float fitness = n / tot[17].x;
-    const bool became_best = rsme < lowest;  // kokkosICP.cpp:181-185
+    asm volatile("bar.sync 2, 64;" ::: "memory");
+    const bool became_best = better != 0;
     if (became_best && lane < 16) st->best[lane] = tn;
     if (out) {  // the final iteration, with a host-mapped result
         if (lane < 16) out->best[lane] = became_best ? tn : st->best[lane];
-        if (lane == 0) out->lowest = became_best ? rsme : lowest;
+        if (lane == 0) out->lowest = low;
     }
-    if (lane != 0) return;
-    if (became_best) st->lowest = rsme;
-    const int it = st->iteration;
-    if (fitness > st->best_fitness) st->best_fitness = fitness;
-    if (it < kIcpIters) {
-        st->stats[it * 4 + 0] = n;
-        st->stats[it * 4 + 1] = rsme;
-        st->stats[it * 4 + 2] = fitness;
-        st->stats[it * 4 + 3] = became_best ? 1.f : 0.f;
-    }
-    st->iteration = it + 1;
-    st->ticket = 0;
-    st->overflow = 0;
 }
 
 // The iteration kernel's grid: one CTA per 32 x 16 tile of source pixels.
