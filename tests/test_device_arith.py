@@ -38,3 +38,66 @@ def test_depth_quotient_is_the_ieee_division_for_every_u16():
     lo = (q0d - (hi - bb)) + (p - bb)  # TwoSum: hi + lo == q0 + p exactly
     got = _rn32_exact(hi, lo)
     assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+# ------------------------------------------------ the voxel index shortcuts
+
+F = np.float32
+
+
+def _fma32(a, b, c):
+    """fma(a, b, c) of float32 values to within the double rounding of a float64 sum (the margins tested below
+    are compared against quantities that far larger steps separate)."""
+    return (a.astype(np.float64) * np.float64(b) + np.float64(c)).astype(F)
+
+
+def _idx_rule(a, length):
+    q = a / F(length)
+    return np.where(a >= 0, np.trunc(q), np.trunc(q - F(1))).astype(np.int64)
+
+
+def _round_parts(a, rlen):
+    """(floor of q, |q - rint(q)|, |q|) with q = RN(a rlen), as the kernels take them from 1.5 2^23 added and taken off."""
+    q = a * F(rlen)
+    t = q + F(12582912.0)
+    d = q - (t - F(12582912.0))
+    return (t.view(np.int32) - np.int32(0x4B400000) + (d.view(np.int32) >> 31)).astype(np.int64), np.abs(d), np.abs(q)
+
+
+def _points(length, rng):
+    """Coordinates over the packable range, most within a room, many within a few ulp of a voxel boundary."""
+    lim = 8191 * 8 * float(length)
+    u = np.concatenate([rng.uniform(-4, 4, 200_000), rng.uniform(-lim, lim, 100_000)]).astype(F)
+    k = np.concatenate([rng.integers(-1200, 1200, 150_000), rng.integers(-65000, 65000, 50_000)])
+    near = (k.astype(np.float64) * float(F(length))).astype(F)
+    for _ in range(3):
+        near = np.concatenate([near, np.nextafter(near[-len(k):], F(np.inf)), np.nextafter(near[:len(k)], F(-np.inf))])
+    j = (k.astype(np.float64) * float(F(length)) * (1 + rng.uniform(-1e-5, 1e-5, len(k)))).astype(F)
+    return np.concatenate([u, near, j, F([0.0, -0.0, 1e-30, -1e-30])])
+
+
+def test_index_shortcuts_give_the_reference_rules():
+    """idx_fast (ss_internal.cuh) and voxel_fast (ss_raycast.cu): where their tests are decisive, the block by
+    idx_rule and the voxel by idx_rule of p - vbl block are those of the shortcut; and they are decisive for all but a
+    few points of a room."""
+    rng = np.random.default_rng(12)
+    for length in (0.004, 0.005, 0.0061, 0.01, 0.02, 1.0 / 128):
+        vl = F(length)
+        vbl = F(8) * vl
+        rvl, rvbl = F(1) / vl, F(1) / vbl
+        p = _points(vl, rng)
+        block = _idx_rule(p, vbl)
+        b, d, q = _round_parts(p, rvbl)
+        ok = d > _fma32(q, F(3.0e-7), F(3.0e-7))
+        assert np.array_equal(b[ok], block[ok])
+        w = p - vbl * block.astype(F)
+        voxel = _idx_rule(w, vl)
+        v, d, q = _round_parts(p, rvl)
+        ok = d > _fma32(q, F(8.0e-7), F(1.6e-5))
+        assert np.array_equal(v[ok] >> 3, block[ok]) and np.array_equal(v[ok] & 7, voxel[ok])
+        assert ok[:200_000].mean() > 0.99
+        bad = F([np.inf, -np.inf, np.nan, 3e9, -3e9])  # never decisive
+        with np.errstate(invalid="ignore", over="ignore"):
+            for r, m, c in ((rvbl, 3.0e-7, 3.0e-7), (rvl, 8.0e-7, 1.6e-5)):
+                _, d, q = _round_parts(bad, r)
+                assert not (d > _fma32(q, F(m), F(c))).any()
