@@ -131,17 +131,21 @@ template <int kStorage>
 __device__ __forceinline__ float refine_crossing(const GridView &g, float ox, float oy, float oz, float dx, float dy,
                                                  float dz, float ta, float fa, float tb, float fb, BlockCache &cache) {
     const float inv_vl = 1.f / g.vl;
+    bool ok = true;
+#pragma unroll 1
     for (int r = 0; r < 2; r++) {
         const float tc = ta + (tb - ta) * fa / (fa - fb);
-        const TriSample q =
-            trilinear<kStorage, false>(g, fmaf(tc, dx, ox), fmaf(tc, dy, oy), fmaf(tc, dz, oz), inv_vl, cache);
-        if (!q.valid) break;
-        if (q.f > 0.f) {
-            ta = tc;
-            fa = q.f;
-        } else {
-            tb = tc;
-            fb = q.f;
+        if (ok) {
+            const TriSample q =
+                trilinear<kStorage, false>(g, fmaf(tc, dx, ox), fmaf(tc, dy, oy), fmaf(tc, dz, oz), inv_vl, cache);
+            ok = q.valid;
+            if (ok && q.f > 0.f) {
+                ta = tc;
+                fa = q.f;
+            } else if (ok) {
+                tb = tc;
+                fb = q.f;
+            }
         }
     }
     return ta + (tb - ta) * fa / (fa - fb);
@@ -179,10 +183,14 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
     float ta = 0.f, fa = 0.f, tb = 0.f, fb = 0.f;  // bracket: f(ta) > 0 > f(tb)
     int csx = INT_MIN, csy = INT_MIN, csz = INT_MIN;
     bool cocc = false;
-    while (steps < max_steps) {
-        if (mode == kRayForward && !(t < t_hi)) break;
+    // one condition ends the loop and no branch inside leaves it: lanes that
+    // took such a branch's other side (a skip instead of a sample) would rejoin
+    // their warp only behind the loop
+    bool go = steps < max_steps && (mode != kRayForward || t < t_hi);
+    while (go) {
         const float px = fmaf(t, dx, ox), py = fmaf(t, dy, oy), pz = fmaf(t, dz, oz);
         steps++;
+        bool skip = false;
         if (mode == kRayForward) {
             const int bx = (int)floorf(px * inv_vbl), by = (int)floorf(py * inv_vbl), bz = (int)floorf(pz * inv_vbl);
             const int sx = bx >> kSuperShift, sy = by >> kSuperShift, sz = bz >> kSuperShift;
@@ -194,7 +202,8 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
                 cache.lookups++;
             }
             const bool empty_super = !cocc;
-            if (empty_super || cached_lookup(g, cache, bx, by, bz) < 0) {
+            skip = empty_super || cached_lookup(g, cache, bx, by, bz) < 0;
+            if (skip) {
                 // exit of the empty super-block's (or block's) box along the ray
                 const float box = empty_super ? sbl : g.vbl;
                 const int cx = empty_super ? sx : bx, cy = empty_super ? sy : by, cz = empty_super ? sz : bz;
@@ -205,33 +214,35 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
                                        dz != 0.f ? ez : INFINITY);
                 t = fmaxf(te, t) + 1e-4f * vl * inv_len;
                 prev_valid = false;
-                continue;
             }
         }
-        const TriSample sm = trilinear<kStorage, false>(g, px, py, pz, inv_vl, cache);
-        if (mode == kRayForward) {
-            if (!sm.valid) {
-                prev_valid = false;
-                t += vl * inv_len;
-                continue;
-            }
-            if (sm.f < 0.f) {
-                found = prev_valid && f_prev > 0.f;  // else a back face
-                ta = t_prev;
-                fa = f_prev;
-                tb = t;
-                fb = sm.f;
-                break;
-            }
-            prev_valid = true;
-            t_prev = t;
-            f_prev = sm.f;
-            t += fmaxf(vl, 0.8f * sm.f) * inv_len;
-        } else if (mode == kRaySeek) {
-            if (!sm.valid) break;  // unobserved at the hint (a gap in the band): no hit
-            t_prev = t;
-            f_prev = sm.f;
-            if (sm.f >= 0.f) {
+        bool end = false;
+        if (!skip) {
+            const TriSample sm = trilinear<kStorage, false>(g, px, py, pz, inv_vl, cache);
+            const bool neg = sm.f < 0.f, pos = sm.f > 0.f;
+            const float step = fmaxf(vl, 0.8f * fabsf(sm.f));  // of a valid sample, in metres
+            if (mode == kRayForward) {
+                if (!sm.valid) {
+                    prev_valid = false;
+                    t += vl * inv_len;
+                } else if (neg) {
+                    found = prev_valid && f_prev > 0.f;  // else a back face
+                    ta = t_prev;
+                    fa = f_prev;
+                    tb = t;
+                    fb = sm.f;
+                    end = true;
+                } else {
+                    prev_valid = true;
+                    t_prev = t;
+                    f_prev = sm.f;
+                    t = fmaf(step, inv_len, t);
+                }
+            } else if (!sm.valid) {
+                end = true;  // unobserved at the hint (a gap in the band) or on the way back: no hit
+            } else if (mode == kRaySeek && sm.f >= 0.f) {
+                t_prev = t;
+                f_prev = sm.f;
                 mode = kRayForward;
                 prev_valid = true;
                 // a valid sample's corner blocks exist, so the super-block of its
@@ -242,27 +253,23 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
                 csy = (int)floorf(py * inv_vbl) >> kSuperShift;
                 csz = (int)floorf(pz * inv_vbl) >> kSuperShift;
                 cocc = true;
-                t += fmaxf(vl, 0.8f * sm.f) * inv_len;
-            } else {
-                mode = kBack;
-                t -= fmaxf(vl, -0.8f * sm.f) * inv_len;
-                if (t < t_lo) break;
-            }
-        } else {  // back
-            if (sm.valid && sm.f > 0.f) {
+                t = fmaf(step, inv_len, t);
+            } else if (mode == kBack && pos) {
                 found = true;
                 ta = t;
                 fa = sm.f;
                 tb = t_prev;
                 fb = f_prev;
-                break;
+                end = true;
+            } else {  // back from a sample behind the surface
+                mode = kBack;
+                t_prev = t;
+                f_prev = sm.f;
+                t = fmaf(-step, inv_len, t);
+                end = t < t_lo;
             }
-            if (!sm.valid) break;
-            t_prev = t;
-            f_prev = sm.f;
-            t -= fmaxf(vl, -0.8f * sm.f) * inv_len;
-            if (t < t_lo) break;
         }
+        go = !end && steps < max_steps && (mode != kRayForward || t < t_hi);
     }
     if (found) t = refine_crossing<kStorage>(g, ox, oy, oz, dx, dy, dz, ta, fa, tb, fb, cache);
     return found;
