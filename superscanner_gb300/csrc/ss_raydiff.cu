@@ -35,34 +35,26 @@ struct CellSample {
     bool valid;
     float f, g[3], Hxy, Hxz, Hyz;
     float a, b, c;  // fractional position in the cell (x, y, z)
-    int bucket[8], vox[8];
+    int ix, iy, iz; // the cell's lowest voxel
 };
 
-// Trilinear value, gradient and Hessian of the cell holding p, with the
-// corners' addresses (for the scatter of voxel gradients).
+// Trilinear value, gradient and Hessian of the cell holding p: the corners by
+// the march's own path (all eight loads in flight; the last cell's values
+// kept, and most Newton steps stay in it).
 template <int kStorage>
 __device__ __forceinline__ void cell_sample(const GridView &g, float px, float py, float pz, float inv_vl,
                                             BlockCache &cache, CellSample &cs) {
     cs.valid = false;
     const float ux = fmaf(px, inv_vl, -0.5f), uy = fmaf(py, inv_vl, -0.5f), uz = fmaf(pz, inv_vl, -0.5f);
     const float fx0 = floorf(ux), fy0 = floorf(uy), fz0 = floorf(uz);
-    const int ix = (int)fx0, iy = (int)fy0, iz = (int)fz0;
+    cs.ix = (int)fx0;
+    cs.iy = (int)fy0;
+    cs.iz = (int)fz0;
     cs.a = ux - fx0;
     cs.b = uy - fy0;
     cs.c = uz - fz0;
     float s[8];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int vx = ix + (k & 1), vy = iy + ((k >> 1) & 1), vz = iz + (k >> 2);
-        const int b = cached_lookup(g, cache, vx >> 3, vy >> 3, vz >> 3);
-        if (b < 0) return;
-        const int v = (vx & 7) + 8 * (vy & 7) + 64 * (vz & 7);
-        const float2 sw = voxel_sw<kStorage>(g, b, v);
-        if (!(sw.y > 0.f)) return;
-        s[k] = sw.x;
-        cs.bucket[k] = b;
-        cs.vox[k] = v;
-    }
+    if (!cell_corners<kStorage>(g, cs.ix, cs.iy, cs.iz, cache, s)) return;
     const float a = cs.a, bb = cs.b, c = cs.c;
     float f = 0.f, ga = 0.f, gb = 0.f, gc = 0.f, hab = 0.f, hac = 0.f, hbc = 0.f;
 #pragma unroll
@@ -117,21 +109,15 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
         cs.valid = false;
         if (hit) {
             // Newton steps to the root of the trilinear field (bounded, safeguarded)
-            for (int it = 0; it < 6; it++) {
+            bool go = true;
+#pragma unroll 1
+            for (int it = 0; it < 6 && go; it++) {
                 cell_sample<kStorage>(g, fmaf(t, dx, ox), fmaf(t, dy, oy), fmaf(t, dz, oz), inv_vl, cache, cs);
-                if (!cs.valid) break;
                 const float gd = cs.g[0] * dx + cs.g[1] * dy + cs.g[2] * dz;
-                if (!(gd < 0.f)) {
-                    cs.valid = false;
-                    break;
-                }
                 const float dt = -cs.f / gd;
-                if (fabsf(dt) > 2.f * g.vl * inv_len) {
-                    cs.valid = false;
-                    break;
-                }
-                t += dt;
-                if (fabsf(dt) < 1e-7f * t) break;
+                cs.valid = cs.valid && gd < 0.f && !(fabsf(dt) > 2.f * g.vl * inv_len);
+                if (cs.valid) t += dt;
+                go = cs.valid && !(fabsf(dt) < 1e-7f * t);
             }
             if (cs.valid) cell_sample<kStorage>(g, fmaf(t, dx, ox), fmaf(t, dy, oy), fmaf(t, dz, oz), inv_vl, cache, cs);
         }
@@ -170,6 +156,8 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
                     }
                     if (grad_vox) {
                         const float ca = cs.a, cb = cs.b, cc = cs.c;
+                        int bk[8];
+                        cell_buckets(g, cs.ix, cs.iy, cs.iz, cache, bk);  // all there: the sample is valid
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
                             const float wx = (k & 1) ? ca : 1.f - ca, wy = ((k >> 1) & 1) ? cb : 1.f - cb;
@@ -178,7 +166,7 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
                             const float sz = (k >> 2) ? 1.f : -1.f;
                             const float mdw = (m[0] * sx * wy * wz + m[1] * wx * sy * wz + m[2] * wx * wy * sz) * inv_vl;
                             const float gk = -e * (wx * wy * wz) + b * mdw;
-                            atomicAdd(grad_vox + (size_t)cs.bucket[k] * kBlockVoxels + cs.vox[k], gk);
+                            atomicAdd(grad_vox + (size_t)bk[k] * kBlockVoxels + cell_voxel(cs.ix, cs.iy, cs.iz, k), gk);
                         }
                     }
                 }

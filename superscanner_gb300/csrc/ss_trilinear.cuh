@@ -52,63 +52,79 @@ __device__ __forceinline__ int block_find(const GridView &g, BlockCache &c, int 
     return packable(bx, by, bz) ? table_find(g, prime_hash(bx, by, bz)) : -1;
 }
 
+// The buckets of the blocks that hold the 8 corners of the cell with lowest
+// voxel (ix, iy, iz), corner k = a + 2 b + 4 c; false where one is missing. One
+// lookup of the cell's lowest block, and, for a cell straddling block faces,
+// one find of each further block (corner (a, b, c) lies in block offset
+// (a sx, b sy, c sz)).
+__device__ __forceinline__ bool cell_buckets(const GridView &g, int ix, int iy, int iz, BlockCache &c, int *bk) {
+    const int bx0 = ix >> 3, by0 = iy >> 3, bz0 = iz >> 3;
+    const bool sx = (ix & 7) == 7, sy = (iy & 7) == 7, sz = (iz & 7) == 7;
+    bk[0] = cached_lookup(g, c, bx0, by0, bz0);
+    if (bk[0] < 0) return false;
+#pragma unroll
+    for (int k = 1; k < 8; k++) bk[k] = bk[0];
+    if (sx | sy | sz) {
+        if (sx) bk[1] = block_find(g, c, bx0 + 1, by0, bz0);
+        if (sy) bk[2] = block_find(g, c, bx0, by0 + 1, bz0);
+        if (sz) bk[4] = block_find(g, c, bx0, by0, bz0 + 1);
+        bk[3] = (sx && sy) ? block_find(g, c, bx0 + 1, by0 + 1, bz0) : (sx ? bk[1] : bk[2]);
+        bk[5] = (sx && sz) ? block_find(g, c, bx0 + 1, by0, bz0 + 1) : (sx ? bk[1] : bk[4]);
+        bk[6] = (sy && sz) ? block_find(g, c, bx0, by0 + 1, bz0 + 1) : (sy ? bk[2] : bk[4]);
+        bk[7] = (sx && sy && sz) ? block_find(g, c, bx0 + 1, by0 + 1, bz0 + 1)
+                                 : (sx && sy ? bk[3] : (sx && sz ? bk[5] : (sy && sz ? bk[6] : (sx ? bk[1] : (sy ? bk[2] : bk[4])))));
+    }
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 8; k++) ok &= bk[k] >= 0;
+    return ok;
+}
+
+// The voxel of corner k in its block.
+__device__ __forceinline__ int cell_voxel(int ix, int iy, int iz, int k) {
+    const int vx = ix + (k & 1), vy = iy + ((k >> 1) & 1), vz = iz + (k >> 2);
+    return (vx & 7) + 8 * (vy & 7) + 64 * (vz & 7);
+}
+
+// The cell's 8 corner values; false where a corner is missing or unobserved.
+// The last cell's are kept. One code path for cells in one block and cells
+// that straddle, so that the corner loads of a warp whose lanes hold both
+// kinds are issued together.
+template <int kStorage>
+__device__ __forceinline__ bool cell_corners(const GridView &g, int ix, int iy, int iz, BlockCache &c, float *s) {
+    if (ix == c.cx && iy == c.cy && iz == c.cz) {  // same cell as the last sample: its corners again
+        if (!c.cok) return false;
+#pragma unroll
+        for (int k = 0; k < 8; k++) s[k] = c.cs[k];
+        return true;
+    }
+    c.cx = ix, c.cy = iy, c.cz = iz, c.cok = false;
+    int bk[8];
+    if (!cell_buckets(g, ix, iy, iz, c, bk)) return false;
+    bool ok = true;
+    float2 sw[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) sw[k] = voxel_sw<kStorage>(g, bk[k], cell_voxel(ix, iy, iz, k));
+    c.voxels += 8;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        ok &= sw[k].y > 0.f;
+        s[k] = sw[k].x;
+        c.cs[k] = s[k];
+    }
+    c.cok = ok;
+    return ok;
+}
+
 template <int kStorage, bool kGrad>
 __device__ __forceinline__ TriSample trilinear(const GridView &g, float px, float py, float pz, float inv_vl,
                                                BlockCache &c) {
     TriSample r{false, 0.f, 0.f, 0.f, 0.f};
     const float ux = fmaf(px, inv_vl, -0.5f), uy = fmaf(py, inv_vl, -0.5f), uz = fmaf(pz, inv_vl, -0.5f);
     const float fx0 = floorf(ux), fy0 = floorf(uy), fz0 = floorf(uz);
-    const int ix = (int)fx0, iy = (int)fy0, iz = (int)fz0;
     const float ax = ux - fx0, ay = uy - fy0, az = uz - fz0;
     float s[8];
-    if (ix == c.cx && iy == c.cy && iz == c.cz) {  // same cell as the last sample: its corners again
-        if (!c.cok) return r;
-#pragma unroll
-        for (int k = 0; k < 8; k++) s[k] = c.cs[k];
-    } else {
-        // The cell's 8 corners: one lookup of the cell's lowest block, and,
-        // for a cell straddling block faces, one find of each further block
-        // (corner (a, b, c) lies in block offset (a sx, b sy, c sz)). One code
-        // path for both kinds of cell, so that the corner loads of a warp
-        // whose lanes hold both kinds are issued together.
-        c.cx = ix, c.cy = iy, c.cz = iz, c.cok = false;
-        const int bx0 = ix >> 3, by0 = iy >> 3, bz0 = iz >> 3;
-        const bool sx = (ix & 7) == 7, sy = (iy & 7) == 7, sz = (iz & 7) == 7;
-        int bk[8];
-        bk[0] = cached_lookup(g, c, bx0, by0, bz0);
-        if (bk[0] < 0) return r;
-#pragma unroll
-        for (int k = 1; k < 8; k++) bk[k] = bk[0];
-        if (sx | sy | sz) {
-            if (sx) bk[1] = block_find(g, c, bx0 + 1, by0, bz0);
-            if (sy) bk[2] = block_find(g, c, bx0, by0 + 1, bz0);
-            if (sz) bk[4] = block_find(g, c, bx0, by0, bz0 + 1);
-            bk[3] = (sx && sy) ? block_find(g, c, bx0 + 1, by0 + 1, bz0) : (sx ? bk[1] : bk[2]);
-            bk[5] = (sx && sz) ? block_find(g, c, bx0 + 1, by0, bz0 + 1) : (sx ? bk[1] : bk[4]);
-            bk[6] = (sy && sz) ? block_find(g, c, bx0, by0 + 1, bz0 + 1) : (sy ? bk[2] : bk[4]);
-            bk[7] = (sx && sy && sz) ? block_find(g, c, bx0 + 1, by0 + 1, bz0 + 1)
-                                     : (sx && sy ? bk[3] : (sx && sz ? bk[5] : (sy && sz ? bk[6] : (sx ? bk[1] : (sy ? bk[2] : bk[4])))));
-        }
-        bool ok = true;
-#pragma unroll
-        for (int k = 0; k < 8; k++) ok &= bk[k] >= 0;
-        if (!ok) return r;
-        float2 sw[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int vx = ix + (k & 1), vy = iy + ((k >> 1) & 1), vz = iz + (k >> 2);
-            sw[k] = voxel_sw<kStorage>(g, bk[k], (vx & 7) + 8 * (vy & 7) + 64 * (vz & 7));
-        }
-        c.voxels += 8;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            ok &= sw[k].y > 0.f;
-            s[k] = sw[k].x;
-            c.cs[k] = s[k];
-        }
-        c.cok = ok;
-        if (!ok) return r;
-    }
+    if (!cell_corners<kStorage>(g, (int)fx0, (int)fy0, (int)fz0, c, s)) return r;
     // lerp along x, then y, then z
     const float s00 = fmaf(ax, s[1] - s[0], s[0]), s10 = fmaf(ax, s[3] - s[2], s[2]);
     const float s01 = fmaf(ax, s[5] - s[4], s[4]), s11 = fmaf(ax, s[7] - s[6], s[6]);
