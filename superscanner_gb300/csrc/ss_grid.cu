@@ -597,6 +597,7 @@ ss_status ss_grid_destroy(ss_grid *g) {
     cudaFree((void *)g->v.ray_v);
     cudaFree(g->phase_mask);
     cudaFree(g->mesh_count);
+    cudaFree(g->t_hit);
     cudaFree(g->batch_poses);
     cudaFree((void *)g->batch_depths);
     delete g;

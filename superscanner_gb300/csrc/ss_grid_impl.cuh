@@ -24,6 +24,7 @@ struct ss_grid {
     ss::FramePose *batch_poses = nullptr;  // [kMaxPhases]
     const uint16_t **batch_depths = nullptr;  // [kMaxPhases / 2] device pointers
     unsigned long long *mesh_count = nullptr;  // triangle counter of ss_grid_extract_mesh (first call)
+    float *t_hit = nullptr;                // [resi][resj] hit depths of the differentiable raycast (first call)
     // launch collect, fuse and raycast as programmatic dependents of the kernel
     // before them (set by the per-frame pipeline while it captures its graph)
     bool pdl = false;

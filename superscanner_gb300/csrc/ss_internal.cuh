@@ -189,21 +189,11 @@ static __device__ __noinline__ int idx_rule(float a, float len) {
 // RN(q1 - 1), and the truncations agree; both are then floor(q1) (a >= 0:
 // q1 >= 0 is no integer; a < 0: neither is RN(q1 - 1), which truncates to
 // floor(q1)). idx_fast returns false where q1 is too close to an integer (and
-// for zero, huge or non-finite values): there the IEEE division decides. The
-// nearest integer comes from adding 1.5 2^23 (its low bits) and taking it off
-// again, two FP32 additions instead of two conversions on the slow pipe (from
-// 2^22 on, where it is off, the margin is above the distance it can show).
+// for zero, huge or non-finite values): there the IEEE division decides.
 __device__ __forceinline__ bool idx_fast(float a, float rlen, int &out) {
     const float q1 = __fmul_rn(a, rlen);
-    const float t = __fadd_rn(q1, 12582912.f), d = __fsub_rn(q1, __fsub_rn(t, 12582912.f));
-    out = __float_as_int(t) - 0x4B400000 + (__float_as_int(d) >> 31);
-    return fabsf(d) > __fmaf_rn(fabsf(q1), 3.0e-7f, 3.0e-7f);  // > 5 u (|q1| + 1)
-}
-
-// idx_rule(a, len) through idx_fast where that is decisive (rlen = RN(1 / len)).
-__device__ __forceinline__ int idx_rule_fast(float a, float len, float rlen) {
-    int o;
-    return idx_fast(a, rlen, o) ? o : idx_rule(a, len);
+    out = __float2int_rd(q1);
+    return fabsf(__fsub_rn(q1, rintf(q1))) > __fmaf_rn(fabsf(q1), 3.0e-7f, 3.0e-7f);  // > 5 u (|q1| + 1)
 }
 
 // The block range of a point's truncation band: idx_rule of its corners lo
@@ -231,8 +221,8 @@ __device__ __forceinline__ unsigned long long prime_hash(int x, int y, int z) {
 }
 
 __device__ __forceinline__ bool packable(int x, int y, int z) {
-    return x >= -kCoordBias && x < kCoordBias && y >= -kCoordBias && y < kCoordBias && z >= -kCoordBias &&
-           z < kCoordBias;
+    return (((unsigned)(x + kCoordBias) | (unsigned)(y + kCoordBias) | (unsigned)(z + kCoordBias)) &
+            ~(2u * kCoordBias - 1u)) == 0u;
 }
 __device__ __forceinline__ unsigned long long pack_coords(int x, int y, int z) {
     return ((unsigned long long)(uint32_t)(x + kCoordBias) << 28) |

@@ -30,6 +30,27 @@ __device__ __forceinline__ VoxelRead read_voxel(const GridView &g, int bucket, i
     }
 }
 
+// floor(q) and |q - rint(q)| of q = RN(p rlen), the nearest integer by adding
+// 1.5 2^23 (its low bits) and taking it off again: FP32 additions, whose
+// latency a march of dependent steps sees, instead of two conversions (the
+// block collection, bound by its instructions, keeps the conversions). From
+// 2^22 on, where the nearest integer is off, the callers' margins exceed the
+// distance it can show.
+__device__ __forceinline__ float floor_and_distance(float p, float rlen, float &q, int &out) {
+    q = __fmul_rn(p, rlen);
+    const float t = __fadd_rn(q, 12582912.f), d = __fsub_rn(q, __fsub_rn(t, 12582912.f));
+    out = __float_as_int(t) - 0x4B400000 + (__float_as_int(d) >> 31);
+    return fabsf(d);
+}
+
+// idx_rule(a, len) by idx_fast's test where that is decisive (rlen = RN(1 / len)).
+__device__ __forceinline__ int idx_rule_fast(float a, float len, float rlen) {
+    float q;
+    int o;
+    const float d = floor_and_distance(a, rlen, q, o);
+    return d > __fmaf_rn(fabsf(q), 3.0e-7f, 3.0e-7f) ? o : idx_rule(a, len);
+}
+
 // getVBIndeces (GPUVoxelGrid.h:162-189): the index rule of each coordinate
 // (by multiplication where that is provably the IEEE quotient's result).
 __device__ __forceinline__ void block_of(const GridView &g, F3 p, int &bx, int &by, int &bz) {
@@ -56,9 +77,9 @@ __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, i
 // asks q for 13 u |q| + 268 u. Elsewhere (one point in a thousand at 2 m and 4 mm
 // voxels) the two rules decide one after the other.
 __device__ __forceinline__ bool voxel_fast(float p, float rvl, int &out) {
-    const float q = __fmul_rn(p, rvl), t = __fadd_rn(q, 12582912.f), d = __fsub_rn(q, __fsub_rn(t, 12582912.f));
-    out = __float_as_int(t) - 0x4B400000 + (__float_as_int(d) >> 31);
-    return fabsf(d) > __fmaf_rn(fabsf(q), 8.0e-7f, 1.6e-5f);
+    float q;
+    const float d = floor_and_distance(p, rvl, q, out);
+    return d > __fmaf_rn(fabsf(q), 8.0e-7f, 1.6e-5f);
 }
 static __device__ __noinline__ int4 voxel_slow(float px, float py, float pz, float vl, float rvl, float vbl, float rvbl) {
     const int bx = idx_rule_fast(px, vbl, rvbl), by = idx_rule_fast(py, vbl, rvbl), bz = idx_rule_fast(pz, vbl, rvbl);
@@ -448,7 +469,8 @@ __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 
     if (hit) {
         const float px = fmaf(t, dx, ox), py = fmaf(t, dy, oy), pz = fmaf(t, dz, oz);
         const TriSample q = trilinear<kStorage, true>(g, px, py, pz, inv_vl, cache);
-        const float gn = q.valid ? sqrtf(q.gx * q.gx + q.gy * q.gy + q.gz * q.gz) : 0.f;
+        // the sum's order is written out: a compiler's choice of it would move the normal's last bit
+        const float gn = q.valid ? sqrtf(fmaf(q.gz, q.gz, fmaf(q.gy, q.gy, __fmul_rn(q.gx, q.gx)))) : 0.f;
         if (gn > 0.f) {
             v = make_float4(px, py, pz, t);
             n = make_float4(q.gx / gn, q.gy / gn, q.gz / gn, 0.f);

@@ -80,9 +80,35 @@ __device__ __forceinline__ void cell_sample(const GridView &g, float px, float p
     cs.valid = true;
 }
 
+// The march of every pixel's ray: its hit depth into t_hit, NaN for a miss. A
+// kernel of its own: the loss kernel sums a CTA's 256 pixels in the order of
+// the image rows, and with the march inside it a CTA's fast warps waited there
+// for its slowest (SMs active 71 % of the launch); here nothing waits, and a
+// warp marches an 8 x 4 patch of rays.
+constexpr int kMarchWarps = 4;  // a CTA's, side by side: a 32 x 4 pixel tile
+template <int kStorage>
+__global__ void __launch_bounds__(32 * kMarchWarps) raymarch_kernel(GridView g, Mat34 T, int max_steps, float t_min,
+                                                                    float t_max, float *__restrict__ t_hit) {
+    const int ln = threadIdx.x & 31;
+    const int j = blockIdx.x * (8 * kMarchWarps) + (threadIdx.x >> 5) * 8 + (ln & 7), i = blockIdx.y * 4 + (ln >> 3);
+    if (i < g.resi && j < g.resj) {
+        const float dcx = ((float)j - g.in.cj) / g.in.fx, dcy = ((float)i - g.in.ci) / g.in.fy;
+        const float dx = fmaf(T.m[0], dcx, fmaf(T.m[1], dcy, T.m[2]));
+        const float dy = fmaf(T.m[4], dcx, fmaf(T.m[5], dcy, T.m[6]));
+        const float dz = fmaf(T.m[8], dcx, fmaf(T.m[9], dcy, T.m[10]));
+        const float inv_len = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
+        BlockCache cache{INT_MIN, INT_MIN, INT_MIN, -1, 0u, 0u};
+        int steps = 0;
+        float t = t_min;
+        const bool hit = march<kStorage>(g, T.m[3], T.m[7], T.m[11], dx, dy, dz, inv_len, t_min, t_max, max_steps,
+                                         steps, t, cache);
+        t_hit[(size_t)i * g.resj + j] = hit ? t : __int_as_float(0x7fc00000);
+    }
+}
+
 template <int kStorage, bool kBackward>
 __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const uint16_t *__restrict__ obs,
-                                                      int max_steps, float t_min, float t_max, float lambda_n,
+                                                      const float *__restrict__ t_hit, float lambda_n,
                                                       float r_max, unsigned long long *__restrict__ facc,
                                                       double *result, int *ticket,
                                                       float *__restrict__ grad_vox,
@@ -102,12 +128,13 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
         const float inv_len = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
         const float inv_vl = 1.f / g.vl;
         BlockCache cache{INT_MIN, INT_MIN, INT_MIN, -1, 0u, 0u};
-        int steps = 0;
-        float t = t_min;
-        bool hit = march<kStorage>(g, ox, oy, oz, dx, dy, dz, inv_len, t_min, t_max, max_steps, steps, t, cache);
+        const size_t pix = (size_t)i * g.resj + j;
+        const float d_obs = (float)__ldg(obs + pix) * 1e-3f;
+        pdl_wait();  // the march's hits
+        float t = __ldcg(t_hit + pix);
         CellSample cs;
         cs.valid = false;
-        if (hit) {
+        if (t == t) {  // a hit
             // Newton steps to the root of the trilinear field (bounded, safeguarded)
             bool go = true;
 #pragma unroll 1
@@ -121,9 +148,7 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
             }
             if (cs.valid) cell_sample<kStorage>(g, fmaf(t, dx, ox), fmaf(t, dy, oy), fmaf(t, dz, oz), inv_vl, cache, cs);
         }
-        const size_t pix = (size_t)i * g.resj + j;
         if (depth_out) depth_out[pix] = cs.valid ? t : 0.f;
-        const float d_obs = (float)__ldg(obs + pix) * 1e-3f;
         if (cs.valid && d_obs > g.rmin && (!mask || __ldg(mask + pix))) {
             const float gn = sqrtf(cs.g[0] * cs.g[0] + cs.g[1] * cs.g[1] + cs.g[2] * cs.g[2]);
             const float n[3] = {cs.g[0] / gn, cs.g[1] / gn, cs.g[2] / gn};
@@ -157,7 +182,9 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
                     if (grad_vox) {
                         const float ca = cs.a, cb = cs.b, cc = cs.c;
                         int bk[8];
-                        cell_buckets(g, cs.ix, cs.iy, cs.iz, cache, bk);  // all there: the sample is valid
+                        // all there: the sample is valid
+                        cell_finds(g, cached_lookup(g, cache, cs.ix >> 3, cs.iy >> 3, cs.iz >> 3), cs.ix, cs.iy, cs.iz,
+                                   cell_straddle(cs.ix, cs.iy, cs.iz), cache, bk);
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
                             const float wx = (k & 1) ? ca : 1.f - ca, wy = ((k >> 1) & 1) ? cb : 1.f - cb;
@@ -273,13 +300,30 @@ static ss_status raydiff(ss_grid *g, const double T[16], const uint16_t *obs, fl
     if (st != SS_OK) return st;
     const Mat34 M = mat34_from(Tf);
     const float t_min = g->p.rmin, t_max = g->p.d_max;
+    if (!g->t_hit && cudaMalloc(&g->t_hit, (size_t)g->p.resi * g->p.resj * sizeof(float)) != cudaSuccess) {
+        cudaGetLastError();
+        g->t_hit = nullptr;
+        return SS_ERR_NOMEM;
+    }
+    const dim3 mgrid((g->p.resj + 8 * kMarchWarps - 1) / (8 * kMarchWarps), (g->p.resi + 3) / 4);
+    if (g->p.storage == SS_STORAGE_F32)
+        raymarch_kernel<SS_STORAGE_F32><<<mgrid, 32 * kMarchWarps, 0, s>>>(g->v, M, max_steps, t_min, t_max, g->t_hit);
+    else
+        raymarch_kernel<SS_STORAGE_F16><<<mgrid, 32 * kMarchWarps, 0, s>>>(g->v, M, max_steps, t_min, t_max, g->t_hit);
+    SS_LAUNCH_CHECK();
 #define SS_RD(ST, BW)                                                                                           \
-    raydiff_kernel<ST, BW><<<grid, blk, 0, s>>>(g->v, M, obs, max_steps, t_min, t_max, lambda_n, r_max, d->facc, \
-                                                d->result_mapped, d->ticket, grad_vox, depth_out, mask)
+    SS_CUDA_TRY(launch_kernel(raydiff_kernel<ST, BW>, grid, blk, 0, s, true, g->v, M, obs, (const float *)g->t_hit, \
+                              lambda_n, r_max, d->facc, d->result_mapped, d->ticket, grad_vox, depth_out, mask))
     if (g->p.storage == SS_STORAGE_F32) {
-        if (backward) SS_RD(SS_STORAGE_F32, true); else SS_RD(SS_STORAGE_F32, false);
+        if (backward)
+            SS_RD(SS_STORAGE_F32, true);
+        else
+            SS_RD(SS_STORAGE_F32, false);
     } else {
-        if (backward) SS_RD(SS_STORAGE_F16, true); else SS_RD(SS_STORAGE_F16, false);
+        if (backward)
+            SS_RD(SS_STORAGE_F16, true);
+        else
+            SS_RD(SS_STORAGE_F16, false);
     }
 #undef SS_RD
     SS_LAUNCH_CHECK();

@@ -52,31 +52,31 @@ __device__ __forceinline__ int block_find(const GridView &g, BlockCache &c, int 
     return packable(bx, by, bz) ? table_find(g, prime_hash(bx, by, bz)) : -1;
 }
 
-// The buckets of the blocks that hold the 8 corners of the cell with lowest
-// voxel (ix, iy, iz), corner k = a + 2 b + 4 c; false where one is missing. One
-// lookup of the cell's lowest block, and, for a cell straddling block faces,
-// one find of each further block (corner (a, b, c) lies in block offset
-// (a sx, b sy, c sz)).
-__device__ __forceinline__ bool cell_buckets(const GridView &g, int ix, int iy, int iz, BlockCache &c, int *bk) {
-    const int bx0 = ix >> 3, by0 = iy >> 3, bz0 = iz >> 3;
-    const bool sx = (ix & 7) == 7, sy = (iy & 7) == 7, sz = (iz & 7) == 7;
-    bk[0] = cached_lookup(g, c, bx0, by0, bz0);
-    if (bk[0] < 0) return false;
+// The axes along which the cell with lowest voxel (ix, iy, iz) straddles a
+// block face, as bits 1 (x), 2 (y), 4 (z): corner k = a + 2 b + 4 c lies in the
+// block at offset bits k & cell_straddle from the cell's lowest block.
+__device__ __forceinline__ int cell_straddle(int ix, int iy, int iz) {
+    return ((ix & 7) == 7 ? 1 : 0) | ((iy & 7) == 7 ? 2 : 0) | ((iz & 7) == 7 ? 4 : 0);
+}
+
+// The corners' buckets bk of a cell whose lowest block has bucket `base`; false
+// where one is missing. A straddling cell's further blocks (1, 3 or 7) are
+// found one a turn, each lane its own next one: lanes that straddle along
+// different axes share the turns (a branch per block cost a warp all seven).
+__device__ __forceinline__ bool cell_finds(const GridView &g, int base, int ix, int iy, int iz, int straddle,
+                                           BlockCache &c, int *bk) {
 #pragma unroll
-    for (int k = 1; k < 8; k++) bk[k] = bk[0];
-    if (sx | sy | sz) {
-        if (sx) bk[1] = block_find(g, c, bx0 + 1, by0, bz0);
-        if (sy) bk[2] = block_find(g, c, bx0, by0 + 1, bz0);
-        if (sz) bk[4] = block_find(g, c, bx0, by0, bz0 + 1);
-        bk[3] = (sx && sy) ? block_find(g, c, bx0 + 1, by0 + 1, bz0) : (sx ? bk[1] : bk[2]);
-        bk[5] = (sx && sz) ? block_find(g, c, bx0 + 1, by0, bz0 + 1) : (sx ? bk[1] : bk[4]);
-        bk[6] = (sy && sz) ? block_find(g, c, bx0, by0 + 1, bz0 + 1) : (sy ? bk[2] : bk[4]);
-        bk[7] = (sx && sy && sz) ? block_find(g, c, bx0 + 1, by0 + 1, bz0 + 1)
-                                 : (sx && sy ? bk[3] : (sx && sz ? bk[5] : (sy && sz ? bk[6] : (sx ? bk[1] : (sy ? bk[2] : bk[4])))));
-    }
+    for (int k = 0; k < 8; k++) bk[k] = base;
     bool ok = true;
+    int m = (0 - straddle) & straddle;  // the first non-empty subset of the straddled axes
+    while (m) {
+        const int b = block_find(g, c, (ix >> 3) + (m & 1), (iy >> 3) + ((m >> 1) & 1), (iz >> 3) + (m >> 2));
 #pragma unroll
-    for (int k = 0; k < 8; k++) ok &= bk[k] >= 0;
+        for (int k = 1; k < 8; k++)
+            if ((k & straddle) == m) bk[k] = b;
+        ok &= b >= 0;
+        m = ok ? (m - straddle) & straddle : 0;  // the next subset
+    }
     return ok;
 }
 
@@ -99,8 +99,9 @@ __device__ __forceinline__ bool cell_corners(const GridView &g, int ix, int iy, 
         return true;
     }
     c.cx = ix, c.cy = iy, c.cz = iz, c.cok = false;
+    const int base = cached_lookup(g, c, ix >> 3, iy >> 3, iz >> 3);
     int bk[8];
-    if (!cell_buckets(g, ix, iy, iz, c, bk)) return false;
+    if (base < 0 || !cell_finds(g, base, ix, iy, iz, cell_straddle(ix, iy, iz), c, bk)) return false;
     bool ok = true;
     float2 sw[8];
 #pragma unroll

@@ -77,7 +77,7 @@ def _points(length, rng):
 
 
 def test_index_shortcuts_give_the_reference_rules():
-    """idx_fast (ss_internal.cuh) and voxel_fast (ss_raycast.cu): where their tests are decisive, the block by
+    """idx_fast (ss_internal.cuh), idx_rule_fast and voxel_fast (ss_raycast.cu): where their tests are decisive, the block by
     idx_rule and the voxel by idx_rule of p - vbl block are those of the shortcut; and they are decisive for all but a
     few points of a room."""
     rng = np.random.default_rng(12)
