@@ -23,7 +23,7 @@ struct ss_grid {
     uint32_t *phase_mask = nullptr;        // [buckets][kMaxPhases / 32]
     ss::FramePose *batch_poses = nullptr;  // [kMaxPhases]
     const uint16_t **batch_depths = nullptr;  // [kMaxPhases / 2] device pointers
-    unsigned long long *mesh_count = nullptr;  // triangle counter of ss_grid_extract_mesh (first call)
+    unsigned long long *mesh_count = nullptr;  // triangle and bucket counters of mesh extraction (first call)
     float *t_hit = nullptr;                // [resi][resj] hit depths of the differentiable raycast (first call)
     // launch collect, fuse and raycast as programmatic dependents of the kernel
     // before them (set by the per-frame pipeline while it captures its graph)
