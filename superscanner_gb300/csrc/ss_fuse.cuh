@@ -8,66 +8,130 @@
 
 namespace ss {
 
-// One voxel of integrationCore[Color]Tag / deIntegrationCore[Color]Tag
-// (GPUVoxelGrid.cpp:345-469, 516-550) in the reference's arithmetic. Returns
-// true when the voxel changes; pixel (cori, corj) and the observed sdf come
-// back through the references.
-__device__ __forceinline__ bool voxel_observe(const GridView &g, const uint16_t *__restrict__ depth, const Mat34 &E,
-                                              const Mat34 &Einv, const F3 &Ez, F3 vm, float &sdf, int &pix) {
-    const F3 q = xform(Einv, vm);
-    const float c0 = __fadd_rn(__fdiv_rn(__fmul_rn(q.y, g.in.fy), q.z), g.in.ci);  // getCoordinate (GPUVoxelGrid.h:234-237)
-    const float c1 = __fadd_rn(__fdiv_rn(__fmul_rn(q.x, g.in.fx), q.z), g.in.cj);
-    // the reference's (int) cast (GPUVoxelGrid.cpp:348-349), which picks the pixel half a pixel off the projection
-    const int cori = __float2int_rz(c0);
-    const int corj = __float2int_rz(c1);
-    if (!(cori < g.resi && corj < g.resj && cori >= 0 && corj >= 0)) return false;
-    pix = cori * g.resj + corj;
-    F3 vpt = get_point(g.in, cori, corj, depth_m(__ldg(depth + pix)));
-    if (!(vpt.z > g.rmin)) return false;
-    vpt = xform(E, vpt);
-    sdf = f3dot(f3sub(vpt, vm), Ez);
-    return fabsf(sdf) < g.trunc;
+// The pixel a voxel projects to (getCoordinate, GPUVoxelGrid.h:234-237, and the
+// reference's (int) cast, GPUVoxelGrid.cpp:348-349, which picks the pixel half
+// a pixel off the projection), in the reference's arithmetic.
+static __device__ __noinline__ int project_axis(float p, float f, float z, float c) {
+    return __float2int_rz(__fadd_rn(__fdiv_rn(__fmul_rn(p, f), z), c));
 }
 
-// The fast path's observation of a voxel from its camera-frame point q =
-// Einv vm: the nearest pixel (the reference's truncation picks the pixel half
-// a pixel off the projection, which makes frame-to-model tracking drift),
-// within the image, with the half pixel of the rounding folded into the
-// principal point and the projection from an approximate reciprocal (the
-// pixel choice only needs it to ~1 ulp); its depth d > rmin; and the
-// projective sdf d - q.z within the truncation: for a rigid E, (E p - vm) . Ez
-// with p the pixel's point at depth d is d - q.z, the distance along the
-// camera axis (a voxel behind the camera gets d + |q.z| > trunc).
-__device__ __forceinline__ bool observe_fast(const GridView &g, const uint16_t *__restrict__ depth, F3 q, float &sdf,
-                                             int &pix) {
-    float rz;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rz) : "f"(q.z));
-    const int cori = __float2int_rd(fmaf(q.y * g.in.fy, rz, g.in.ci + 0.5f));
-    const int corj = __float2int_rd(fmaf(q.x * g.in.fx, rz, g.in.cj + 0.5f));
-    if (!(cori < g.resi && corj < g.resj && cori >= 0 && corj >= 0)) return false;
-    pix = cori * g.resj + corj;
-    const float d = (float)__ldg(depth + pix) * 1.0e-3f;
-    if (!(d > g.rmin)) return false;
-    sdf = d - q.z;
-    return fabsf(sdf) < g.trunc;
+// The same with the quotient from an approximate reciprocal (1 ulp) where that
+// decides the pixel: the approximate coordinate a and the reference's lie
+// within 3 u |p f / z| + 2 u |a| of each other (u = 2^-24), so where a is
+// further than 4e-7 (|a| + |c|) from every integer they truncate alike (|p f / z|
+// <= |a| + |c| and its roundings). Elsewhere (one coordinate in a thousand at
+// 640 x 480), and for zero, infinite and NaN depths, the division decides.
+__device__ __forceinline__ int project_axis_fast(float p, float f, float z, float rz, float c) {
+    const float a = fmaf(__fmul_rn(p, f), rz, c);
+    return fabsf(a - rintf(a)) > __fmul_rn(4.0e-7f, fabsf(a) + fabsf(c)) ? __float2int_rz(a) : project_axis(p, f, z, c);
 }
 
-// Camera-frame points of a lane's four voxels r0 .. r0 + 3 (r0 even: voxel
-// (l0, m0) of vm0, then (l0 + 4, m0), (l0, m0 + 1), (l0 + 4, m0 + 1)) for the
-// fast path: the first as Einv vm0, the others by adding the transformed
-// voxel steps (4 vl along y, vl along z), with rounded operations that are
-// never contracted, so every kernel computes the same values (the per-frame
-// fusion and the batched re-fusion stay bit-identical).
-__device__ __forceinline__ void quad_points_fast(const Mat34 &Einv, F3 vm0, float vl, F3 q[4]) {
-    q[0].x = fmaf(vm0.x, Einv.m[0], fmaf(vm0.y, Einv.m[1], fmaf(vm0.z, Einv.m[2], Einv.m[3])));
-    q[0].y = fmaf(vm0.x, Einv.m[4], fmaf(vm0.y, Einv.m[5], fmaf(vm0.z, Einv.m[6], Einv.m[7])));
-    q[0].z = fmaf(vm0.x, Einv.m[8], fmaf(vm0.y, Einv.m[9], fmaf(vm0.z, Einv.m[10], Einv.m[11])));
+// The observation of integrationCore[Color]Tag / deIntegrationCore[Color]Tag
+// (GPUVoxelGrid.cpp:345-469, 516-550) of a lane's four voxels (rows r0 .. r0 +
+// 3 of the block at pz: voxel (k, l0 + 4 (r & 1), r >> 1) at row r) in the
+// reference's arithmetic: whether a voxel changes, its pixel and observed sdf.
+// The four depth gathers are in flight together.
+__device__ __forceinline__ void quad_observe_exact(const GridView &g, const uint16_t *__restrict__ depth, const Mat34 &E,
+                                                   const Mat34 &Einv, const F3 &Ez, F3 vm0, F3 pz, int l0, int r0,
+                                                   float obs[4], bool ok[4], int pix[4]) {
+    auto centre = [&](int rr) {
+        const int l = l0 + 4 * (rr & 1), m = (r0 + rr) >> 1;
+        return F3{vm0.x, __fmaf_rn((float)l + 0.5f, g.vl, pz.y), __fmaf_rn((float)m + 0.5f, g.vl, pz.z)};
+    };
+    uint16_t d[4];
+    float u[4], v[4];
+#pragma unroll
+    for (int rr = 0; rr < 4; rr++) {
+        const F3 q = xform(Einv, centre(rr));
+        float rz;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rz) : "f"(q.z));
+        const int i = project_axis_fast(q.y, g.in.fy, q.z, rz, g.in.ci), j = project_axis_fast(q.x, g.in.fx, q.z, rz, g.in.cj);
+        ok[rr] = (unsigned)i < (unsigned)g.resi && (unsigned)j < (unsigned)g.resj;
+        pix[rr] = i * g.resj + j;
+        d[rr] = ok[rr] ? __ldg(depth + pix[rr]) : (uint16_t)0;
+        u[rr] = ok[rr] ? __ldg(g.ray_u + j) : 0.f;
+        v[rr] = ok[rr] ? __ldg(g.ray_v + i) : 0.f;
+    }
+#pragma unroll
+    for (int rr = 0; rr < 4; rr++) {
+        const float z = depth_m(d[rr]);
+        const F3 p = xform(E, F3{__fmul_rn(u[rr], z), __fmul_rn(v[rr], z), z});  // getPoint from the grid's quotients
+        obs[rr] = f3dot(f3sub(p, centre(rr)), Ez);
+        ok[rr] = ok[rr] && z > g.rmin && fabsf(obs[rr]) < g.trunc;
+    }
+}
+
+// The fast path's observation of a voxel whose pixel holds `depth`: d > rmin,
+// and the projective sdf d - q.z within the truncation (q = Einv vm): for a
+// rigid E, (E p - vm) . Ez with p the pixel's point at depth d is d - q.z, the
+// distance along the camera axis (a voxel behind the camera gets d + |q.z| >
+// trunc).
+__device__ __forceinline__ bool observe_fast(const GridView &g, uint16_t depth, float qz, float &sdf) {
+    // (float)depth: 2^23 + depth, the 2^23 taken off again
+    const float d = (__uint_as_float(0x4B000000u | depth) - 8388608.f) * 1.0e-3f;
+    sdf = d - qz;
+    return d > g.rmin && fabsf(sdf) < g.trunc;
+}
+
+// The fast path's observation of a lane's four voxels r0 .. r0 + 3 (r0 even:
+// voxel (l0, m0) at vm0, then (l0 + 4, m0), (l0, m0 + 1), (l0 + 4, m0 + 1)).
+// Camera-frame points: Einv vm0 and, for the others, the transformed voxel
+// steps (4 vl along y, vl along z) added with rounded operations that are
+// never contracted. Pixels: the nearest (the reference's truncation picks the
+// pixel half a pixel off the projection, which makes frame-to-model tracking
+// drift), with the half pixel of the rounding folded into the principal point
+// and the projection from an approximate reciprocal (the pixel choice only
+// needs it to ~1 ulp); the floors come from additions of 1.5 2^23 rounded down:
+// an integer below 2^22 in the sum's low bits, and for everything else
+// (infinities and NaN too) a number outside any image. Voxels 0 and 2, then 1
+// and 3 go through paired instructions (the same roundings); the four gathers
+// are in flight together, and no branch comes before they have arrived. The
+// per-frame fusion and the batched re-fusion share it (bit for bit the same
+// volume).
+__device__ __forceinline__ void quad_observe_fast(const GridView &g, const uint16_t *__restrict__ depth,
+                                                  const Mat34 &Einv, F3 vm0, float vl, float obs[4], bool ok[4],
+                                                  int pix[4]) {
+    const float ax = fmaf(vm0.x, Einv.m[0], fmaf(vm0.y, Einv.m[1], fmaf(vm0.z, Einv.m[2], Einv.m[3])));
+    const float ay = fmaf(vm0.x, Einv.m[4], fmaf(vm0.y, Einv.m[5], fmaf(vm0.z, Einv.m[6], Einv.m[7])));
+    const float az = fmaf(vm0.x, Einv.m[8], fmaf(vm0.y, Einv.m[9], fmaf(vm0.z, Einv.m[10], Einv.m[11])));
     const float sy = __fmul_rn(4.f, vl);
-    const F3 dy{__fmul_rn(Einv.m[1], sy), __fmul_rn(Einv.m[5], sy), __fmul_rn(Einv.m[9], sy)};
-    const F3 dz{__fmul_rn(Einv.m[2], vl), __fmul_rn(Einv.m[6], vl), __fmul_rn(Einv.m[10], vl)};
-    q[1] = F3{__fadd_rn(q[0].x, dy.x), __fadd_rn(q[0].y, dy.y), __fadd_rn(q[0].z, dy.z)};
-    q[2] = F3{__fadd_rn(q[0].x, dz.x), __fadd_rn(q[0].y, dz.y), __fadd_rn(q[0].z, dz.z)};
-    q[3] = F3{__fadd_rn(q[2].x, dy.x), __fadd_rn(q[2].y, dy.y), __fadd_rn(q[2].z, dy.z)};
+    auto both = [](float v) { return f2_pack(v, v); };
+    f32x2 x[2], y[2], z[2];  // voxels (0, 2) and (1, 3)
+    x[0] = f2_pack(ax, __fadd_rn(ax, __fmul_rn(Einv.m[2], vl)));
+    y[0] = f2_pack(ay, __fadd_rn(ay, __fmul_rn(Einv.m[6], vl)));
+    z[0] = f2_pack(az, __fadd_rn(az, __fmul_rn(Einv.m[10], vl)));
+    x[1] = f2_add(x[0], both(__fmul_rn(Einv.m[1], sy)));
+    y[1] = f2_add(y[0], both(__fmul_rn(Einv.m[5], sy)));
+    z[1] = f2_add(z[0], both(__fmul_rn(Einv.m[9], sy)));
+    uint16_t d[4];
+    float qz[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        float r[2], fi[2], fj[2];
+        f2_unpack(z[h], qz[h], qz[h + 2]);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[0]) : "f"(qz[h]));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[1]) : "f"(qz[h + 2]));
+        const f32x2 rz = f2_pack(r[0], r[1]), big = both(12582912.f);
+        f2_unpack(f2_add_down(f2_fma(f2_mul(y[h], both(g.in.fy)), rz, both(g.in.ci + 0.5f)), big), fi[0], fi[1]);
+        f2_unpack(f2_add_down(f2_fma(f2_mul(x[h], both(g.in.fx)), rz, both(g.in.cj + 0.5f)), big), fj[0], fj[1]);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const unsigned i = __float_as_uint(fi[u]) - 0x4B400000u, j = __float_as_uint(fj[u]) - 0x4B400000u;
+            pix[h + 2 * u] = (int)(i * (unsigned)g.resj + j);
+            ok[h + 2 * u] = i < (unsigned)g.resi && j < (unsigned)g.resj;
+            d[h + 2 * u] = ok[h + 2 * u] ? __ldg(depth + pix[h + 2 * u]) : (uint16_t)0;
+        }
+    }
+#pragma unroll
+    for (int rr = 0; rr < 4; rr++) ok[rr] = observe_fast(g, d[rr], qz[rr], obs[rr]) && ok[rr];
+}
+
+// x / y for a weight y (1 .. 2^24): x times the approximate reciprocal, as
+// __fdividef gives it there without its steps for denormal and huge y.
+__device__ __forceinline__ float div_weight(float x, float y) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    return x * r;
 }
 
 // Running-average update of one voxel (sdf, weight) in FP32.
@@ -75,12 +139,12 @@ template <bool kDeint, bool kExact>
 __device__ __forceinline__ void running_average(float &s, float &w, float obs, float max_weight) {
     if (!kDeint) {
         const float w1 = kExact ? __fadd_rn(w, 1.f) : w + 1.f;
-        s = kExact ? __fdiv_rn(__fadd_rn(__fmul_rn(s, w), obs), w1) : __fdividef(fmaf(s, w, obs), w1);
+        s = kExact ? __fdiv_rn(__fadd_rn(__fmul_rn(s, w), obs), w1) : div_weight(fmaf(s, w, obs), w1);
         w = (max_weight > 0.f && w1 > max_weight) ? max_weight : w1;
     } else {
         if (w != 1.f) {
             const float w1 = kExact ? __fsub_rn(w, 1.f) : w - 1.f;
-            s = kExact ? __fdiv_rn(__fsub_rn(__fmul_rn(s, w), obs), w1) : __fdividef(fmaf(s, w, -obs), w1);
+            s = kExact ? __fdiv_rn(__fsub_rn(__fmul_rn(s, w), obs), w1) : div_weight(fmaf(s, w, -obs), w1);
             w = w1;
         } else {
             w = 0.f;

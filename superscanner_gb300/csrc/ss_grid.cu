@@ -160,11 +160,16 @@ __global__ void __launch_bounds__(256, 8) collect_kernel(GridView g, const uint1
 // Voxel centres: the reference computes pzero + (k + 0.5) * vl in double and
 // rounds to float (GPUVoxelGrid.cpp:521); that double sum is exact for
 // |pzero| < 2^20 m, so one fmaf (single rounding of the exact value) gives the
-// identical float. Registers are capped at 32 (8 CTAs, 64 warps per SM: the
-// kernel waits on dependent loads, and the few spilled bytes cost less than
-// the lost occupancy; 0.0164 -> 0.0154 ms per frame).
+// identical float. A lane's four observations come first, their depth gathers
+// together (ss_fuse.cuh), then the updates. The fast path's registers are
+// capped at 32 (8 CTAs, 64 warps per SM: the kernel waits on dependent loads;
+// 16.0 -> 12.7 us for a frame of 1280 x 720). The reference's arithmetic holds
+// more values between the gathers and the updates: 48 registers (5 CTAs; FP16
+// 517 x 389 20 -> 17 us, 19 us at 32), and with colour, whose twelve plane
+// values and pixel bytes are loaded together too, 64 (4 CTAs; FP32 640 x 480 50
+// -> 36 us; 40 at 48 and 39 at 77).
 template <int kStorage, bool kColor, bool kDeint, bool kExact>
-__global__ void __launch_bounds__(256, 8) fuse_kernel(GridView g, const uint16_t *__restrict__ depth,
+__global__ void __launch_bounds__(256, kColor ? 4 : kExact ? 5 : 8) fuse_kernel(GridView g, const uint16_t *__restrict__ depth,
                                                    const uint8_t *__restrict__ rgb, Mat34 E, Mat34 Einv, F3 Ez,
                                                    const FramePose *__restrict__ pose) {
     pdl_wait();     // the block list (collection) and the pose (tracker)
@@ -199,22 +204,35 @@ __global__ void __launch_bounds__(256, 8) fuse_kernel(GridView g, const uint16_t
         const float pzx = __fmul_rn(g.vbl, (float)bx), pzy = __fmul_rn(g.vbl, (float)by),
                     pzz = __fmul_rn(g.vbl, (float)bz);
         const float cx = __fmaf_rn((float)k + 0.5f, g.vl, pzx);
-        F3 qf[4];  // fast path: the four camera-frame points (ss_fuse.cuh)
-        if (!kExact)
-            quad_points_fast(Einv, F3{cx, __fmaf_rn((float)l0 + 0.5f, g.vl, pzy), __fmaf_rn((float)(r0 >> 1) + 0.5f, g.vl, pzz)},
-                             g.vl, qf);
+        const F3 vm0{cx, __fmaf_rn((float)l0 + 0.5f, g.vl, pzy), __fmaf_rn((float)(r0 >> 1) + 0.5f, g.vl, pzz)};
+        float obs4[4];
+        bool ok[4];
+        int pix4[4];
+        if (kExact)
+            quad_observe_exact(g, depth, E, Einv, Ez, vm0, F3{pzx, pzy, pzz}, l0, r0, obs4, ok, pix4);
+        else
+            quad_observe_fast(g, depth, Einv, vm0, g.vl, obs4, ok, pix4);
+        // the colours of the voxels that change, and their pixels', all in flight together
+        float col[4][3];
+        uint8_t seen[4][3];
+        if (kColor) {
+#pragma unroll
+            for (int rr = 0; rr < 4; rr++) {
+                const float *pl = g.rgb + (size_t)bucket * 3 * kBlockVoxels + lane + 32 * (r0 + rr);
+                const uint8_t *c = rgb + (size_t)pix4[rr] * 3;
+#pragma unroll
+                for (int ch = 0; ch < 3; ch++) {
+                    col[rr][ch] = ok[rr] ? pl[ch * kBlockVoxels] : 0.f;
+                    seen[rr][ch] = ok[rr] ? __ldg(c + ch) : (uint8_t)0;
+                }
+            }
+        }
 #pragma unroll
         for (int rr = 0; rr < 4; rr++) {
-            const int r = r0 + rr;
-            const int l = l0 + 4 * (r & 1), m = r >> 1;
-            const int v = lane + 32 * r;  // == k + 8 l + 64 m
-            const F3 vm{cx, __fmaf_rn((float)l + 0.5f, g.vl, pzy), __fmaf_rn((float)m + 0.5f, g.vl, pzz)};
+            if (!ok[rr]) continue;
+            const int v = lane + 32 * (r0 + rr);  // == k + 8 l + 64 m
             const size_t vi = (size_t)bucket * kBlockVoxels + v;
-            float obs;
-            int pix;
-            if (kExact ? !voxel_observe(g, depth, E, Einv, Ez, vm, obs, pix)
-                       : !observe_fast(g, depth, qf[rr], obs, pix))
-                continue;
+            const float obs = obs4[rr];
             float s, w;
             if (kStorage == SS_STORAGE_F32) {
                 s = sw32[rr].x;
@@ -235,12 +253,11 @@ __global__ void __launch_bounds__(256, 8) fuse_kernel(GridView g, const uint16_t
                 g.vox16[vi] = (uint32_t)hs | ((uint32_t)wc << 16);
             }
             if (kColor) {
-                const uint8_t *c = rgb + (size_t)pix * 3;
                 float *pl = g.rgb + (size_t)bucket * 3 * kBlockVoxels + v;
 #pragma unroll
                 for (int ch = 0; ch < 3; ch++) {
-                    float cv = pl[ch * kBlockVoxels];
-                    color_average<kDeint, kExact>(cv, w_old, (float)c[ch]);
+                    float cv = col[rr][ch];
+                    color_average<kDeint, kExact>(cv, w_old, (float)seen[rr][ch]);
                     pl[ch * kBlockVoxels] = cv;
                 }
             }

@@ -408,6 +408,17 @@ __device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
     return r;
 }
 
+__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_add_down(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Exact cross-CTA sums in fixed point (resolution 2^-48): a CTA's float
 // value becomes a signed integer below 2^95 in magnitude, added as three
 // 32-bit chunks (two unsigned, the top one signed) into three 64-bit words

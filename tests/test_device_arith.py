@@ -101,3 +101,23 @@ def test_index_shortcuts_give_the_reference_rules():
             for r, m, c in ((rvbl, 3.0e-7, 3.0e-7), (rvl, 8.0e-7, 1.6e-5)):
                 _, d, q = _round_parts(bad, r)
                 assert not (d > _fma32(q, F(m), F(c))).any()
+
+
+def test_projected_pixel_shortcut_gives_the_reference_cast():
+    """project_axis_fast (ss_fuse.cuh): wherever its test is decisive, for any reciprocal within 1 ulp of 1 / z, the
+    truncated coordinate is that of the reference's IEEE quotient; undecided only near pixel edges."""
+    rng = np.random.default_rng(5)
+    for f, c, n in ((525.0, 319.5, 640), (131.25, 60.5, 120), (2100.0, 1279.5, 4096), (60.0, -3.0, 64)):
+        f, c = F(f), F(c)
+        z = rng.uniform(0.05, 12.0, 400_000).astype(F) * rng.choice([1, 1, 1, -1], 400_000).astype(F)
+        t = rng.uniform(-1.5 * n, 1.5 * n, 400_000)  # the pixel aimed at, a third of them next to an edge
+        t[::3] = np.round(t[::3]) + rng.uniform(-2e-3, 2e-3, len(t[::3]))
+        p = ((t - float(c)) * z.astype(np.float64) / float(f)).astype(F)
+        pf = p * f
+        want = np.trunc(pf / z + c).astype(np.int64)
+        y = (1.0 / z.astype(np.float64)).astype(F)
+        for rz in (y, np.nextafter(y, F(np.inf)), np.nextafter(y, F(-np.inf))):
+            a = (pf.astype(np.float64) * rz.astype(np.float64) + float(c)).astype(F)
+            sure = np.abs(a - np.rint(a)) > F(4.0e-7) * (np.abs(a) + np.abs(c))
+            assert np.array_equal(np.trunc(a).astype(np.int64)[sure], want[sure])
+            assert sure[1::3].mean() > 0.98
