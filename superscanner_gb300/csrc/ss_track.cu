@@ -18,6 +18,8 @@
 // redundantly), or one launch per iteration (CTA slots reduced with TwoSum in
 // a fixed order by the last CTA to finish, which solves). No host
 // synchronisation between iterations, levels or frames.
+#include <algorithm>
+
 #include "ss_grid_impl.cuh"
 #include "ss_track.cuh"
 #include "ss_track_solve.cuh"
@@ -108,6 +110,29 @@ __global__ void pose_prep_kernel(TrackState *st) {
     if (threadIdx.x == 0) write_frame_pose(st->T, &st->pose);
 }
 
+// The pixels tid, tid + nthreads, ... of a level's image one after the other:
+// row and column by one division, then by additions.
+struct PixelWalk {
+    int i, j, di, dj, lc;
+    __device__ __forceinline__ PixelWalk(int p, int step, int cols)
+        : i(p / cols), j(p % cols), di(step / cols), dj(step % cols), lc(cols) {}
+    __device__ __forceinline__ void next() {
+        i += di;
+        j += dj;
+        if (j >= lc) {
+            j -= lc;
+            i++;
+        }
+    }
+};
+
+// x . y and a b - c d with their contractions written out: left to the compiler
+// they differ between the group sizes below, and the pose with them.
+__device__ __forceinline__ float dot3(float x0, float x1, float x2, float y0, float y1, float y2) {
+    return fmaf(x2, y2, fmaf(x0, y0, __fmul_rn(x1, y1)));
+}
+__device__ __forceinline__ float det2(float a, float b, float c, float d) { return fmaf(a, b, -__fmul_rn(c, d)); }
+
 // Accumulates this thread's share of one Gauss-Newton iteration at a level
 // into Kahan (sum, compensation) pairs. The thread's pixels are visited in
 // groups of kTrackGroup: all depth loads of a group, then all model-map loads,
@@ -124,14 +149,16 @@ __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ de
     const int lr = (rows + (1 << level) - 1) >> level, lc = (cols + (1 << level) - 1) >> level;
     const int npix = lr * lc;
     const float rfx = 1.f / in.fx, rfy = 1.f / in.fy;
+    PixelWalk at(tid, nthreads, lc);
     for (int base = tid; base < npix; base += kTrackGroup * nthreads) {
         float d[kTrackGroup];
         int pi[kTrackGroup], pj[kTrackGroup];
 #pragma unroll
         for (int g = 0; g < kTrackGroup; g++) {
             const int p = base + g * nthreads;
-            pi[g] = (p / lc) << level;
-            pj[g] = (p % lc) << level;
+            pi[g] = at.i << level;
+            pj[g] = at.j << level;
+            at.next();
             d[g] = p < npix ? (float)__ldg(depth + (size_t)pi[g] * cols + pj[g]) * 1e-3f : 0.f;
         }
         float wv[kTrackGroup][3];
@@ -174,9 +201,10 @@ __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ de
             if (nn.x == 0.f && nn.y == 0.f && nn.z == 0.f) continue;
             const float wx = wv[g][0], wy = wv[g][1], wz = wv[g][2];
             const float ex = wx - vv.x, ey = wy - vv.y, ez = wz - vv.z;
-            if (ex * ex + ey * ey + ez * ez > dist2) continue;
-            const float r = nn.x * ex + nn.y * ey + nn.z * ez;
-            const float J[6] = {wy * nn.z - wz * nn.y, wz * nn.x - wx * nn.z, wx * nn.y - wy * nn.x, nn.x, nn.y, nn.z};
+            if (dot3(ex, ey, ez, ex, ey, ez) > dist2) continue;
+            const float r = dot3(nn.x, nn.y, nn.z, ex, ey, ez);
+            const float J[6] = {det2(wy, nn.z, wz, nn.y), det2(wz, nn.x, wx, nn.z), det2(wx, nn.y, wy, nn.x),
+                                nn.x, nn.y, nn.z};
             int q = 0;
 #pragma unroll
             for (int a = 0; a < 6; a++)
@@ -197,7 +225,8 @@ __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ de
 
 // The persistent tracker keeps each thread's source points of a level in
 // shared memory across the level's iterations (a pixel's camera-frame point
-// does not depend on the pose): up to kCamCache pixels per thread.
+// does not depend on the pose): up to kCamCache pixels per thread. (24 of them,
+// for the finest level of 1280 x 720, took as long as recomputing the points.)
 constexpr int kCamCache = 8;
 
 // Camera-frame points (x, y, d, valid) of this thread's pixels at a level,
@@ -208,13 +237,14 @@ __device__ __forceinline__ void track_fill_cam(const uint16_t *__restrict__ dept
     const int lc = (cols + (1 << level) - 1) >> level;
     const int npix = ((rows + (1 << level) - 1) >> level) * lc;
     const float rfx = 1.f / in.fx, rfy = 1.f / in.fy;
+    PixelWalk at(tid, nthreads, lc);
 #pragma unroll
-    for (int m = 0; m < kCamCache; m++) {
+    for (int m = 0; m < kCamCache; m++, at.next()) {
         if (m >= m_count) break;
         const int p = tid + m * nthreads;
         float4 cp = make_float4(0.f, 0.f, 0.f, 0.f);
         if (p < npix) {
-            const int i = (p / lc) << level, j = (p % lc) << level;
+            const int i = at.i << level, j = at.j << level;
             const float d = (float)__ldg(depth + (size_t)i * cols + j) * 1e-3f;
             if ((d > rmin) && (d < dmax))
                 cp = make_float4(((float)j - in.cj) * rfx * d, ((float)i - in.ci) * rfy * d, d, 1.f);
@@ -229,7 +259,10 @@ __device__ __forceinline__ void track_fill_cam(const uint16_t *__restrict__ dept
 // sums stay compensated; a group adds at most kG - 1 roundings). With
 // kG = kCamCache the thread's points are one group: every gather of the
 // iteration is in flight at once (one memory round trip), and the pairs are
-// the group's sums with zero compensation.
+// the group's sums with zero compensation. The group is no larger than the
+// thread's share where that is one or two pixels: empty places cost their
+// instructions all the same (640 x 480 135.5 -> 132.4 us a frame, 160 x 120 90
+// -> 73 with only as many CTAs as there are pixels for).
 template <int kG>
 __device__ __forceinline__ void track_accumulate_cam(const float4 (*cam)[256], int m_count, int rows, int cols,
                                                      Intr in, const float4 *__restrict__ vmap,
@@ -276,9 +309,10 @@ __device__ __forceinline__ void track_accumulate_cam(const float4 (*cam)[256], i
             if (nn.x == 0.f && nn.y == 0.f && nn.z == 0.f) continue;
             const float wx = wv[g][0], wy = wv[g][1], wz = wv[g][2];
             const float ex = wx - vv.x, ey = wy - vv.y, ez = wz - vv.z;
-            if (ex * ex + ey * ey + ez * ez > dist2) continue;
-            const float r = nn.x * ex + nn.y * ey + nn.z * ez;
-            const float J[6] = {wy * nn.z - wz * nn.y, wz * nn.x - wx * nn.z, wx * nn.y - wy * nn.x, nn.x, nn.y, nn.z};
+            if (dot3(ex, ey, ez, ex, ey, ez) > dist2) continue;
+            const float r = dot3(nn.x, nn.y, nn.z, ex, ey, ez);
+            const float J[6] = {det2(wy, nn.z, wz, nn.y), det2(wz, nn.x, wx, nn.z), det2(wx, nn.y, wy, nn.x),
+                                nn.x, nn.y, nn.z};
             int q = 0;
 #pragma unroll
             for (int a = 0; a < 6; a++)
@@ -290,6 +324,9 @@ __device__ __forceinline__ void track_accumulate_cam(const float4 (*cam)[256], i
             s[28] += 1.f;  // counts stay exact far below 2^24
             any = true;
         }
+        // (a term that is one product must not be contracted into the addition)
+#pragma unroll
+        for (int q = 0; q < kTrackSums - 1; q++) asm("" : "+f"(t[q]));
         if (kG >= kCamCache) {  // the only group
 #pragma unroll
             for (int q = 0; q < kTrackSums - 1; q++) s[q] = t[q];
@@ -725,6 +762,10 @@ __global__ void __launch_bounds__(256) track_frame_kernel(const uint16_t *__rest
             if (cached)
                 if (m_count > kTrackGroup)
                     track_accumulate_cam<kCamCache>(cam, m_count, rows, cols, in, vmap, nmap, T, P, dist2, s, c);
+                else if (m_count == 1)
+                    track_accumulate_cam<1>(cam, m_count, rows, cols, in, vmap, nmap, T, P, dist2, s, c);
+                else if (m_count == 2)
+                    track_accumulate_cam<2>(cam, m_count, rows, cols, in, vmap, nmap, T, P, dist2, s, c);
                 else
                     track_accumulate_cam<kTrackGroup>(cam, m_count, rows, cols, in, vmap, nmap, T, P, dist2, s, c);
             else
@@ -845,7 +886,10 @@ ss_status launch_track(const TrackLaunch &L, cudaStream_t s) {
         // cooperative launch (all CTAs co-resident, so the grid barrier cannot wait
         // on a CTA that is not running); the attribute form is stream-capturable
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(L.ctas);
+        // no more CTAs than give every pixel of the finest level a thread of its
+        // own (the others would only add zeros to the sums that all wait for)
+        const int ctas = std::min(L.ctas, (rows * cols + 255) / 256);
+        cfg.gridDim = dim3(ctas);
         cfg.blockDim = dim3(256);
         cfg.dynamicSmemBytes = 0;
         cfg.stream = s;
