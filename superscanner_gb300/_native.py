@@ -144,13 +144,14 @@ for _name, (_res, _args) in SIGNATURES.items():
     _fn.argtypes = _args
 
 
+_F32x16, _F64x16 = C.c_float * 16, C.c_double * 16
+
+
 def f32x16(m) -> C.Array:
     import numpy as np
-    a = np.ascontiguousarray(np.asarray(m, dtype=np.float32).reshape(16))
-    return (C.c_float * 16)(*a.tolist())
+    return _F32x16.from_buffer_copy(np.ascontiguousarray(np.asarray(m, dtype=np.float32).reshape(16)))
 
 
 def f64x16(m) -> C.Array:
     import numpy as np
-    a = np.ascontiguousarray(np.asarray(m, dtype=np.float64).reshape(16))
-    return (C.c_double * 16)(*a.tolist())
+    return _F64x16.from_buffer_copy(np.ascontiguousarray(np.asarray(m, dtype=np.float64).reshape(16)))

@@ -20,8 +20,15 @@ from ._native import (SS_STORAGE_F16, SS_STORAGE_F32, SSLaunchConfig, SSParams, 
 _STORAGE = {"f32": SS_STORAGE_F32, "f16": SS_STORAGE_F16}
 
 
+# torch's current stream as its handle, without the Stream object that torch.cuda.current_stream() builds
+# (3.0 -> 0.5 us a call, of the 12 that a small call takes)
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_ptr(stream) -> C.c_void_p:
     if stream is None:
+        if _raw_stream is not None:
+            return C.c_void_p(_raw_stream(torch.cuda.current_device()))
         stream = torch.cuda.current_stream()
     return C.c_void_p(stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream))
 
