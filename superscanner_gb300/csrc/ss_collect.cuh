@@ -2,7 +2,9 @@
 // (depthToPcdTag + vbCollectionTag, GPUVoxelGrid.h:303-307,
 // GPUVoxelGrid.cpp:471-514), shared by the per-call collection
 // (collect_kernel, ss_grid.cu) and the batched re-fusion's
-// (refuse_collect_kernel, ss_refuse.cu). One thread per pixel, two phases:
+// (refuse_collect_kernel, ss_refuse.cu). One thread per pixel. Where the cubes
+// of the tile's pixels lie in a small box (TileBits, nearly always), the tile's
+// blocks are collected as bits of the box; elsewhere in two phases:
 //  1. every pixel's candidates, the cube of blocks its truncation band
 //     overlaps (GPUVoxelGrid.cpp:485-489), go into a shared-memory hash set,
 //     so the tile's candidates are deduplicated on chip: the lanes of a warp
@@ -83,30 +85,254 @@ __device__ __forceinline__ bool tile_point(const GridView &g, const uint16_t *__
     return p.z > g.rmin;
 }
 
-// Phase 1 for a pixel of the tile with camera-frame point p (valid: from
-// tile_point) at pose E (every thread of the CTA calls it; the set, and a
-// tagged set's tags, must be cleared and the CTA synced before; fills of a
-// tagged set may follow one another without a barrier).
-template <bool kTagged, class Visit>
-__device__ __forceinline__ void tile_fill_set(const GridView &g, F3 p, bool valid, const Mat34 &E, unsigned *cset,
-                                              int slots, int cbx, int cby, int cbz, unsigned tag, Visit &visit) {
-    const unsigned FULL = 0xffffffffu;
-    __syncwarp();  // the warp's lanes are done with its cube entries of an earlier fill
-    int lox = 0, loy = 0, loz = 0, nx = 0, ny = 0, nz = 0;
+// The cube of blocks a pixel's truncation band overlaps at pose E
+// (GPUVoxelGrid.cpp:485-489): lowest block and extents, all zero extents for a
+// pixel that takes no part (p, valid: from tile_point) or whose cube is out of
+// range.
+struct TileCube {
+    int lox, loy, loz, nx, ny, nz;
+};
+__device__ __forceinline__ TileCube tile_cube(const GridView &g, F3 p, bool valid, const Mat34 &E) {
+    TileCube c{0, 0, 0, 0, 0, 0};
     if (valid) {
         const F3 pt = xform(E, p);
         const F3 t{g.trunc, g.trunc, g.trunc};
         const F3 lo = f3sub(pt, t), hi = f3add(pt, t);
         int hix, hiy, hiz;
-        block_range(lo, hi, g.vbl, g.rvbl, lox, loy, loz, hix, hiy, hiz);
-        nx = hix - lox + 1;
-        ny = hiy - loy + 1;
-        nz = hiz - loz + 1;
-        if (nx < 1 || ny < 1 || nz < 1 || nx > 8 || ny > 8 || nz > 8) {
+        block_range(lo, hi, g.vbl, g.rvbl, c.lox, c.loy, c.loz, hix, hiy, hiz);
+        c.nx = hix - c.lox + 1;
+        c.ny = hiy - c.loy + 1;
+        c.nz = hiz - c.loz + 1;
+        if (c.nx < 1 || c.ny < 1 || c.nz < 1 || c.nx > 8 || c.ny > 8 || c.nz > 8) {
             atomicOr(&g.ctr->status, kStRange);  // non-finite pose or truncation > 3.5 blocks
-            nx = ny = nz = 0;
+            c.nx = c.ny = c.nz = 0;
         }
     }
+    return c;
+}
+
+// Visits the cnt blocks of a warp's list (packed offsets; tags in the top two
+// bits), appending with one atomic per warp step.
+template <bool kTagged, class Visit>
+__device__ __forceinline__ void tile_visit_list(const GridView &g, const unsigned *wlist, int cnt, int cbx, int cby,
+                                                int cbz, Visit &visit) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    __syncwarp();
+    for (int base = 0; base < cnt; base += 32) {
+        const int e = base + lane;
+        bool append = false;
+        int bucket = -1;
+        if (e < cnt) {
+            const unsigned key = wlist[e];
+            append = visit(cbx + (int)((key >> 20) & 1023u) - kSetOff, cby + (int)((key >> 10) & 1023u) - kSetOff,
+                           cbz + (int)(key & 1023u) - kSetOff, kTagged ? key >> 30 : 1u, bucket);
+        }
+        const unsigned ap = __ballot_sync(FULL, append);
+        if (ap) {
+            const int leader = __ffs(ap) - 1;
+            int b0 = 0;
+            if (lane == leader) b0 = atomicAdd(&g.ctr->list_count, __popc(ap));
+            b0 = __shfl_sync(FULL, b0, leader);
+            if (append) {
+                const int idx = b0 + __popc(ap & lt);
+                if (idx <= (int)g.mask) g.list[idx] = bucket;
+                else atomicOr(&g.ctr->status, kStListOverflow);
+            }
+        }
+    }
+}
+
+// ---- The tile's blocks as bits. The cubes of a tile's pixels mostly lie in a
+// small box: with the box's longest side along 16 words at most (two words a
+// step where the second side is longer than 4) and 4 x 8 or 8 x 8 blocks of the
+// other two sides as a word's bits, a warp ORs its lanes' cubes by one
+// reduction a word, and the tile's blocks are the bits of 32 words in shared
+// memory (per phase, for a re-fusion). Tiles whose box does not fit (depth
+// edges, truncation of many blocks; 2 % of a noisy room's) use the set above.
+// Grouping a warp's equal cubes and entering their blocks in the set took most
+// of the instructions that bound the collection: noise gives a 32-pixel row ten
+// and more distinct cubes. 100 keyframes of 640 x 480 0.99 -> 0.75 ms, a frame of
+// 640 x 480 12.8 -> 10.0 us, of 1280 x 720 36 -> 28.6 us.
+struct TileBits {
+    unsigned box[6];  // lowest x, y, z and 1023 - highest x, y, z: block offsets from the camera's block + kSetOff
+    unsigned wide;    // a cube out of the offsets' range
+    unsigned bits[2][32];
+};
+
+__device__ __forceinline__ void tile_bits_clear(TileBits &t) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    if (tid < 32) t.bits[0][tid] = t.bits[1][tid] = 0u;
+    if (tid < 6) t.box[tid] = 2 * kSetOff;  // empty: lowest > highest
+    if (tid == 6) t.wide = 0u;
+}
+
+// A cube's corners as offsets (10 bits an axis); hi < lo for an empty one.
+struct PackedCube {
+    unsigned lo, hi;
+};
+__device__ __forceinline__ PackedCube tile_pack(const TileCube &c, int cbx, int cby, int cbz, TileBits &t) {
+    PackedCube k{0x3fffffffu, 0u};
+    if (c.nx) {
+        const unsigned x = (unsigned)(c.lox - cbx + kSetOff), y = (unsigned)(c.loy - cby + kSetOff),
+                       z = (unsigned)(c.loz - cbz + kSetOff);
+        if (max(max(x, y), z) < 2u * kSetOff - 8u) {  // so do the highest blocks, fewer than 8 further
+            k.lo = x << 20 | y << 10 | z;
+            k.hi = k.lo + ((unsigned)(c.nx - 1) << 20 | (unsigned)(c.ny - 1) << 10 | (unsigned)(c.nz - 1));
+        } else {
+            t.wide = 1u;
+        }
+    }
+    return k;
+}
+
+// Grows the tile's box by the warp's cubes (of both phases: an empty one gives
+// the lowest corner's 1023s and the highest's zeros, 1023 from the top).
+__device__ __forceinline__ void tile_box(PackedCube k, PackedCube m, TileBits &t) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned mine = 0u;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const int sh = 20 - 10 * a;
+        const unsigned l = __reduce_min_sync(FULL, min((k.lo >> sh) & 1023u, (m.lo >> sh) & 1023u));
+        const unsigned h = __reduce_max_sync(FULL, max((k.hi >> sh) & 1023u, (m.hi >> sh) & 1023u));
+        if (lane == a) mine = l;
+        if (lane == 3 + a) mine = 1023u - h;
+    }
+    if (lane < 6) atomicMin(t.box + lane, mine);
+}
+
+// How the box lies in the words: the axis (0 x, 1 y, 2 z) along the words, and
+// the shifts that take an offset's three axes (word axis, byte axis, bit axis)
+// from a packed corner.
+struct TileLayout {
+    bool fits, empty;
+    int sa, sb, sc;                // shifts of the axes in a packed corner
+    unsigned a0, b0, c0;           // the box's lowest offsets along them
+    int na, two;                   // steps along the words, and words a step - 1
+};
+__device__ __forceinline__ TileLayout tile_layout(const TileBits &t, int cbx, int cby, int cbz) {
+    TileLayout L;
+    const int ex = 1024 - (int)(t.box[0] + t.box[3]), ey = 1024 - (int)(t.box[1] + t.box[4]),
+              ez = 1024 - (int)(t.box[2] + t.box[5]);
+    const int a = ex >= ey && ex >= ez ? 0 : ey >= ez ? 1 : 2, b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+    const int eb = b == 0 ? ex : ey, ec = c == 2 ? ez : ey;
+    L.na = a == 0 ? ex : a == 1 ? ey : ez;
+    L.sa = 20 - 10 * a;
+    L.sb = 20 - 10 * b;
+    L.sc = 20 - 10 * c;
+    L.a0 = t.box[a];
+    L.b0 = t.box[b];
+    L.c0 = t.box[c];
+    L.two = eb > 4 ? 1 : 0;
+    L.empty = ex <= 0 && !t.wide;
+    // a warp lists at most 8 words' blocks (tile_flush_words); every offset from
+    // the camera's block is a packable coordinate
+    constexpr unsigned room = kCoordBias - kSetOff;
+    const bool near = (unsigned)cbx + room <= 2 * room && (unsigned)cby + room <= 2 * room && (unsigned)cbz + room <= 2 * room;
+    L.fits = !t.wide && near && ex > 0 && L.na <= 16 && eb <= 8 && ec <= 8 && (L.na << L.two) <= 8 * (int)blockDim.y;
+    return L;
+}
+
+// ORs the warp's cubes into the words of one phase.
+__device__ __forceinline__ void tile_fill_bits(PackedCube k, const TileLayout &L, unsigned *words) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const bool any = k.hi >= k.lo;
+    const int a0 = any ? (int)(((k.lo >> L.sa) & 1023u) - L.a0) : 31, a1 = any ? (int)(((k.hi >> L.sa) & 1023u) - L.a0) : -1;
+    const unsigned b0 = ((k.lo >> L.sb) & 1023u) - L.b0, nb = ((k.hi >> L.sb) & 1023u) - L.b0 - b0;
+    const unsigned c0 = ((k.lo >> L.sc) & 1023u) - L.c0, nc = ((k.hi >> L.sc) & 1023u) - L.c0 - c0;
+    const unsigned row = any ? ((2u << nc) - 1u) << c0 : 0u;  // a byte's bits
+    const unsigned rows = any ? ((2u << nb) - 1u) << b0 : 0u; // which bytes
+    // a nibble's bits spread to four bytes' lowest, times the byte
+    const unsigned m0 = ((rows & 15u) * 0x00204081u & 0x01010101u) * row;
+    const unsigned m1 = ((rows >> 4) * 0x00204081u & 0x01010101u) * row;
+    const int first = __reduce_min_sync(FULL, a0), last = __reduce_max_sync(FULL, a1);
+    unsigned mine = 0u;
+    for (int a = first; a <= last; a++) {
+        const bool in = a >= a0 && a <= a1;
+        const unsigned o0 = __reduce_or_sync(FULL, in ? m0 : 0u);
+        if (lane == a << L.two) mine = o0;
+        if (L.two) {
+            const unsigned o1 = __reduce_or_sync(FULL, in ? m1 : 0u);
+            if (lane == 2 * a + 1) mine = o1;
+        }
+    }
+    if (mine) atomicOr(words + lane, mine);
+}
+
+// A listed block: bit `lane` of word w, with its tag.
+template <bool kTagged>
+__device__ __forceinline__ unsigned tile_bit_key(const TileLayout &L, int w, int lane, unsigned b0, unsigned b1) {
+    const unsigned ka = L.a0 + (unsigned)(w >> L.two), kb = L.b0 + (L.two ? 4u * (w & 1) : 0u) + (lane >> 3),
+                   kc = L.c0 + (lane & 7);
+    const unsigned tag = kTagged ? ((b0 >> lane) & 1u) | ((b1 >> lane) & 1u) << 1 : 0u;
+    return ka << L.sa | kb << L.sb | kc << L.sc | tag << 30;
+}
+
+// Phase 2 from the bits (after a CTA barrier that follows the fills), list: the
+// set's memory. Two ways to share a tile's blocks among its warps:
+// - one frame, where the latency of the visits counts: warp w lists the blocks
+//   of words w, w + nw, ... and visits them (at most 8 words: 256 entries);
+// - a re-fusion's many tiles, where the instructions count: warp w visits the
+//   tile's blocks 32 w .. 32 w + 31, in the order of the bits, then those 32 nw
+//   further, so that a visit's lanes are full and most warps of a tile have
+//   none (100 keyframes 0.86 -> 0.79 ms, but 1 us more for one 517 x 389 frame).
+template <class Visit>
+__device__ __forceinline__ void tile_flush_words(const GridView &g, const TileBits &t, const TileLayout &L, unsigned *list,
+                                                 int nw, int cbx, int cby, int cbz, Visit &visit) {
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    unsigned *wlist = list + wid * 256;
+    int cnt = 0;
+    for (int w = wid; w < L.na << L.two; w += nw) {
+        const unsigned b = t.bits[0][w];
+        if ((b >> lane) & 1u) wlist[cnt + __popc(b & lt)] = tile_bit_key<false>(L, w, lane, b, 0u);
+        cnt += __popc(b);
+    }
+    tile_visit_list<false>(g, wlist, cnt, cbx, cby, cbz, visit);
+}
+
+template <class Visit>
+__device__ __forceinline__ void tile_flush_tagged(const GridView &g, const TileBits &t, const TileLayout &L, unsigned *list,
+                                                  int nw, int cbx, int cby, int cbz, Visit &visit) {
+    const unsigned FULL = 0xffffffffu;
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int words = L.na << L.two;
+    unsigned *wlist = list + wid * 32;
+    int incl = __popc(t.bits[0][lane] | t.bits[1][lane]);  // words past the last are zero
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(FULL, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int total = __shfl_sync(FULL, incl, 31);
+    for (int first = wid * 32; first < total; first += nw * 32) {
+        __syncwarp();
+        int at = 0;  // the number of the word's first block
+        for (int w = __popc(__ballot_sync(FULL, incl <= first)); w < words && at < first + 32; w++) {
+            at = w ? __shfl_sync(FULL, incl, w - 1) : 0;
+            const unsigned b0 = t.bits[0][w], b1 = t.bits[1][w], b = b0 | b1;
+            const int pos = at + __popc(b & lt) - first;
+            if (((b >> lane) & 1u) && pos >= 0 && pos < 32) wlist[pos] = tile_bit_key<true>(L, w, lane, b0, b1);
+        }
+        tile_visit_list<true>(g, wlist, min(total - first, 32), cbx, cby, cbz, visit);
+    }
+}
+
+// Phase 1 for a pixel of the tile with the cube c of blocks (every thread of
+// the CTA calls it; the set, and a tagged set's tags, must be cleared and the
+// CTA synced before; fills of a tagged set may follow one another without a
+// barrier).
+template <bool kTagged, class Visit>
+__device__ __forceinline__ void tile_fill_set(const GridView &g, const TileCube &c, unsigned *cset, int slots, int cbx,
+                                              int cby, int cbz, unsigned tag, Visit &visit) {
+    const unsigned FULL = 0xffffffffu;
+    __syncwarp();  // the warp's lanes are done with its cube entries of an earlier fill
+    const int lox = c.lox, loy = c.loy, loz = c.loz, nx = c.nx, ny = c.ny, nz = c.nz;
     const int total = nx * ny * nz;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
@@ -215,29 +441,7 @@ __device__ __forceinline__ void tile_flush_set(const GridView &g, unsigned *cset
             wlist[cnt + __popc(b & lt)] = kTagged ? key | tile_tags(cset, slots)[wid * per + r + lane] << 30 : key;
         cnt += __popc(b);
     }
-    __syncwarp();
-    for (int base = 0; base < cnt; base += 32) {
-        const int e = base + lane;
-        bool append = false;
-        int bucket = -1;
-        if (e < cnt) {
-            const unsigned key = wlist[e];
-            append = visit(cbx + (int)((key >> 20) & 1023u) - kSetOff, cby + (int)((key >> 10) & 1023u) - kSetOff,
-                           cbz + (int)(key & 1023u) - kSetOff, kTagged ? key >> 30 : 1u, bucket);
-        }
-        const unsigned ap = __ballot_sync(FULL, append);
-        if (ap) {
-            const int leader = __ffs(ap) - 1;
-            int b0 = 0;
-            if (lane == leader) b0 = atomicAdd(&g.ctr->list_count, __popc(ap));
-            b0 = __shfl_sync(FULL, b0, leader);
-            if (append) {
-                const int idx = b0 + __popc(ap & lt);
-                if (idx <= (int)g.mask) g.list[idx] = bucket;
-                else atomicOr(&g.ctr->status, kStListOverflow);
-            }
-        }
-    }
+    tile_visit_list<kTagged>(g, wlist, cnt, cbx, cby, cbz, visit);
 }
 
 // Find or insert a block, then stamp it with this call's epoch: the first

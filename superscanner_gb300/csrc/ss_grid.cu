@@ -125,9 +125,10 @@ struct CollectVisit {
 __global__ void __launch_bounds__(256, 8) collect_kernel(GridView g, const uint16_t *__restrict__ depth, Mat34 E,
                                                          const FramePose *__restrict__ pose) {
     extern __shared__ unsigned cset[];  // [slots] keys, then [slots] per-warp lists
-    const int slots = kSetSlotsPerRow * blockDim.y;
+    __shared__ TileBits tile;
+    const int slots = kSetSlotsPerRow * blockDim.y, nw = blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthreads = blockDim.x * blockDim.y;
-    for (int q = tid; q < slots; q += nthreads) cset[q] = kSetEmpty;
+    tile_bits_clear(tile);
     // the frame's depth is an input, not an output of the kernel before this one
     F3 p;
     const bool valid = tile_point(g, depth, blockIdx.y * blockDim.y + threadIdx.y, blockIdx.x * 32 + threadIdx.x, p);
@@ -141,12 +142,27 @@ __global__ void __launch_bounds__(256, 8) collect_kernel(GridView g, const uint1
     camera_block(g, E, cbx, cby, cbz);
     SS_CT(0);
     __syncthreads();
-    tile_fill_set<false>(g, p, valid, E, cset, slots, cbx, cby, cbz, 1u, visit);
-    SS_CT(2);
-    pdl_trigger();  // the fuse kernel may launch once every tile has filled its set
+    const TileCube c = tile_cube(g, p, valid, E);
+    const PackedCube k = tile_pack(c, cbx, cby, cbz, tile);
+    tile_box(k, k, tile);
+    SS_CT(1);
     __syncthreads();
-    SS_CT(3);
-    tile_flush_set<false>(g, cset, slots, cbx, cby, cbz, visit);
+    const TileLayout L = tile_layout(tile, cbx, cby, cbz);
+    if (L.fits) {
+        tile_fill_bits(k, L, tile.bits[0]);
+        SS_CT(2);
+        pdl_trigger();  // the fuse kernel may launch once every tile has filled its words
+        __syncthreads();
+        SS_CT(3);
+        tile_flush_words(g, tile, L, cset, nw, cbx, cby, cbz, visit);
+    } else if (!L.empty) {
+        for (int q = tid; q < slots; q += nthreads) cset[q] = kSetEmpty;
+        __syncthreads();
+        tile_fill_set<false>(g, c, cset, slots, cbx, cby, cbz, 1u, visit);
+        pdl_trigger();
+        __syncthreads();
+        tile_flush_set<false>(g, cset, slots, cbx, cby, cbz, visit);
+    }
     SS_CT(4);
 }
 

@@ -52,30 +52,51 @@ __global__ void __launch_bounds__(256, 8) refuse_collect_kernel(GridView g, cons
                                                                 const FramePose *__restrict__ poses,
                                                                 uint32_t *__restrict__ phase_mask) {
     extern __shared__ unsigned cset[];  // [slots] keys, [slots] per-warp lists, cube entries, [slots] tags
-    const int slots = kSetSlotsPerRow * blockDim.y;
+    __shared__ TileBits tile;
+    const int slots = kSetSlotsPerRow * blockDim.y, nw = blockDim.y;
     const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthreads = blockDim.x * blockDim.y;
-    unsigned *tags = tile_tags(cset, slots);
-    for (int q = tid; q < slots; q += nthreads) {
-        cset[q] = kSetEmpty;
-        tags[q] = 0u;
-    }
+    tile_bits_clear(tile);
     const int phase0 = 2 * blockIdx.z;
     F3 p;
     const bool valid =
         tile_point(g, depths[blockIdx.z], blockIdx.y * blockDim.y + threadIdx.y, blockIdx.x * 32 + threadIdx.x, p);
     RefuseVisit visit{g, *(volatile uint32_t *)&g.ctr->epoch, phase_mask, phase0 >> 5, phase0 & 31};
-    Mat34 E;
+    auto cube = [&](int phase) {
+        Mat34 E;
 #pragma unroll
-    for (int k = 0; k < 12; k++) E.m[k] = __ldg(&poses[phase0].E.m[k]);
+        for (int k = 0; k < 12; k++) E.m[k] = __ldg(&poses[phase].E.m[k]);
+        return tile_cube(g, p, valid, E);
+    };
     int cbx, cby, cbz;
-    camera_block(g, E, cbx, cby, cbz);
-    __syncthreads();
-    tile_fill_set<true>(g, p, valid, E, cset, slots, cbx, cby, cbz, 1u, visit);
+    {
+        Mat34 E;
 #pragma unroll
-    for (int k = 0; k < 12; k++) E.m[k] = __ldg(&poses[phase0 + 1].E.m[k]);
-    tile_fill_set<true>(g, p, valid, E, cset, slots, cbx, cby, cbz, 2u, visit);
+        for (int k = 0; k < 12; k++) E.m[k] = __ldg(&poses[phase0].E.m[k]);
+        camera_block(g, E, cbx, cby, cbz);
+    }
     __syncthreads();
-    tile_flush_set<true>(g, cset, slots, cbx, cby, cbz, visit);
+    const PackedCube k0 = tile_pack(cube(phase0), cbx, cby, cbz, tile);
+    const PackedCube k1 = tile_pack(cube(phase0 + 1), cbx, cby, cbz, tile);
+    tile_box(k0, k1, tile);
+    __syncthreads();
+    const TileLayout L = tile_layout(tile, cbx, cby, cbz);
+    if (L.fits) {
+        tile_fill_bits(k0, L, tile.bits[0]);
+        tile_fill_bits(k1, L, tile.bits[1]);
+        __syncthreads();
+        tile_flush_tagged(g, tile, L, cset, nw, cbx, cby, cbz, visit);
+    } else if (!L.empty) {
+        unsigned *tags = tile_tags(cset, slots);
+        for (int q = tid; q < slots; q += nthreads) {
+            cset[q] = kSetEmpty;
+            tags[q] = 0u;
+        }
+        __syncthreads();
+        tile_fill_set<true>(g, cube(phase0), cset, slots, cbx, cby, cbz, 1u, visit);
+        tile_fill_set<true>(g, cube(phase0 + 1), cset, slots, cbx, cby, cbz, 2u, visit);
+        __syncthreads();
+        tile_flush_set<true>(g, cset, slots, cbx, cby, cbz, visit);
+    }
 }
 
 // Instruction-bound: a phase of a quarter block is ~150 warp instructions. Its
@@ -226,7 +247,7 @@ extern "C" ss_status ss_refuse_batch(ss_grid *g, int32_t n, const uint16_t *cons
     SS_CUDA_TRY(cudaMemcpyAsync(g->batch_poses, hp, 2 * n * sizeof(FramePose), cudaMemcpyHostToDevice, s));
     SS_CUDA_TRY(cudaMemcpyAsync(g->batch_depths, depths, n * sizeof(uint16_t *), cudaMemcpyHostToDevice, s));
     SS_CUDA_TRY(cudaMemsetAsync(&g->v.ctr->work, 0, sizeof(int), s));
-    constexpr int kRows = 4;
+    constexpr int kRows = 8;  // a tile of 8 rows holds few more blocks than one of 4 (0.79 -> 0.75 ms per 100 keyframes)
     const dim3 cblk(32, kRows), cgrid((g->p.resj + 31) / 32, (g->p.resi + kRows - 1) / kRows, n);
     refuse_collect_kernel<<<cgrid, cblk, tile_set_bytes(kRows, true), s>>>(g->v, g->batch_depths, g->batch_poses,
                                                                      g->phase_mask);
