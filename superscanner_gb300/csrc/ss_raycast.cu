@@ -415,7 +415,8 @@ __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 
     const int j = blockIdx.x * 32 + threadIdx.x;
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
     const bool inside = i < g.resi && j < g.resj;
-    BlockCache cache{INT_MIN, INT_MIN, INT_MIN, -1, 0u, 0u};
+    __shared__ int buckets[8 * 512];
+    BlockCache cache(buckets, threadIdx.y * 32 + threadIdx.x, blockDim.y * 32);
     int steps = 0;
     bool hit = false;
     SS_RT_NOW(rt0);

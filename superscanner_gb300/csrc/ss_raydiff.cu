@@ -97,7 +97,8 @@ __global__ void __launch_bounds__(32 * kMarchWarps) raymarch_kernel(GridView g, 
         const float dy = fmaf(T.m[4], dcx, fmaf(T.m[5], dcy, T.m[6]));
         const float dz = fmaf(T.m[8], dcx, fmaf(T.m[9], dcy, T.m[10]));
         const float inv_len = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
-        BlockCache cache{INT_MIN, INT_MIN, INT_MIN, -1, 0u, 0u};
+        __shared__ int buckets[8 * 32 * kMarchWarps];
+        BlockCache cache(buckets, threadIdx.x, 32 * kMarchWarps);
         int steps = 0;
         float t = t_min;
         const bool hit = march<kStorage>(g, T.m[3], T.m[7], T.m[11], dx, dy, dz, inv_len, t_min, t_max, max_steps,
@@ -127,7 +128,8 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
         const float ox = T.m[3], oy = T.m[7], oz = T.m[11];
         const float inv_len = rsqrtf(fmaf(dx, dx, fmaf(dy, dy, dz * dz)));
         const float inv_vl = 1.f / g.vl;
-        BlockCache cache{INT_MIN, INT_MIN, INT_MIN, -1, 0u, 0u};
+        __shared__ int buckets[8 * 256];
+        BlockCache cache(buckets, threadIdx.y * 32 + threadIdx.x, 256);
         const size_t pix = (size_t)i * g.resj + j;
         const float d_obs = (float)__ldg(obs + pix) * 1e-3f;
         pdl_wait();  // the march's hits
@@ -181,10 +183,9 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
                     }
                     if (grad_vox) {
                         const float ca = cs.a, cb = cs.b, cc = cs.c;
-                        int bk[8];
-                        // all there: the sample is valid
+                        const int straddle = cell_straddle(cs.ix, cs.iy, cs.iz);  // all there: the sample is valid
                         cell_finds(g, cached_lookup(g, cache, cs.ix >> 3, cs.iy >> 3, cs.iz >> 3), cs.ix, cs.iy, cs.iz,
-                                   cell_straddle(cs.ix, cs.iy, cs.iz), cache, bk);
+                                   straddle, cache);
 #pragma unroll
                         for (int k = 0; k < 8; k++) {
                             const float wx = (k & 1) ? ca : 1.f - ca, wy = ((k >> 1) & 1) ? cb : 1.f - cb;
@@ -193,7 +194,9 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
                             const float sz = (k >> 2) ? 1.f : -1.f;
                             const float mdw = (m[0] * sx * wy * wz + m[1] * wx * sy * wz + m[2] * wx * wy * sz) * inv_vl;
                             const float gk = -e * (wx * wy * wz) + b * mdw;
-                            atomicAdd(grad_vox + (size_t)bk[k] * kBlockVoxels + cell_voxel(cs.ix, cs.iy, cs.iz, k), gk);
+                            atomicAdd(grad_vox + (size_t)cell_bucket(cache, straddle, k) * kBlockVoxels +
+                                          cell_voxel(cs.ix, cs.iy, cs.iz, k),
+                                      gk);
                         }
                     }
                 }

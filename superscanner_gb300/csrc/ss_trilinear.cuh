@@ -15,9 +15,16 @@ struct TriSample {
 };
 
 struct BlockCache {
-    int x, y, z, bucket;
-    unsigned lookups;  // hash-table finds issued (cache misses)
-    unsigned voxels;   // voxel words loaded
+    // this thread's column of a shared-memory table: at [m * stride] the bucket
+    // of the block at offset m (bits 1 x, 2 y, 4 z) from a cell's lowest block
+    // (cell_finds; eight registers picked by comparisons cost a turn of its
+    // loop more than the find)
+    int *tab;
+    int stride;  // threads of the CTA
+    int x = INT_MIN, y = INT_MIN, z = INT_MIN, bucket = -1;  // the last block looked up
+    unsigned lookups = 0u;  // hash-table finds issued (cache misses)
+    unsigned voxels = 0u;   // voxel words loaded
+    __device__ __forceinline__ BlockCache(int *table, int tid, int threads) : tab(table + tid), stride(threads) {}
     // the last sampled cell (its lowest voxel) and its 8 corner values
     int cx = INT_MIN, cy = INT_MIN, cz = INT_MIN;
     bool cok = false;
@@ -59,25 +66,28 @@ __device__ __forceinline__ int cell_straddle(int ix, int iy, int iz) {
     return ((ix & 7) == 7 ? 1 : 0) | ((iy & 7) == 7 ? 2 : 0) | ((iz & 7) == 7 ? 4 : 0);
 }
 
-// The corners' buckets bk of a cell whose lowest block has bucket `base`; false
-// where one is missing. A straddling cell's further blocks (1, 3 or 7) are
+// The buckets of a cell's blocks into the table (corner k's block at offset k &
+// straddle), the lowest one's being `base`; false where one is missing. A
+// straddling cell's further blocks (1, 3 or 7) are
 // found one a turn, each lane its own next one: lanes that straddle along
 // different axes share the turns (a branch per block cost a warp all seven).
 __device__ __forceinline__ bool cell_finds(const GridView &g, int base, int ix, int iy, int iz, int straddle,
-                                           BlockCache &c, int *bk) {
-#pragma unroll
-    for (int k = 0; k < 8; k++) bk[k] = base;
+                                           BlockCache &c) {
+    c.tab[0] = base;
     bool ok = true;
     int m = (0 - straddle) & straddle;  // the first non-empty subset of the straddled axes
     while (m) {
         const int b = block_find(g, c, (ix >> 3) + (m & 1), (iy >> 3) + ((m >> 1) & 1), (iz >> 3) + (m >> 2));
-#pragma unroll
-        for (int k = 1; k < 8; k++)
-            if ((k & straddle) == m) bk[k] = b;
+        c.tab[m * c.stride] = b;
         ok &= b >= 0;
         m = ok ? (m - straddle) & straddle : 0;  // the next subset
     }
     return ok;
+}
+
+// The bucket of corner k's block, after cell_finds.
+__device__ __forceinline__ int cell_bucket(const BlockCache &c, int straddle, int k) {
+    return c.tab[(k & straddle) * c.stride];
 }
 
 // The voxel of corner k in its block.
@@ -100,12 +110,12 @@ __device__ __forceinline__ bool cell_corners(const GridView &g, int ix, int iy, 
     }
     c.cx = ix, c.cy = iy, c.cz = iz, c.cok = false;
     const int base = cached_lookup(g, c, ix >> 3, iy >> 3, iz >> 3);
-    int bk[8];
-    if (base < 0 || !cell_finds(g, base, ix, iy, iz, cell_straddle(ix, iy, iz), c, bk)) return false;
+    const int straddle = cell_straddle(ix, iy, iz);
+    if (base < 0 || !cell_finds(g, base, ix, iy, iz, straddle, c)) return false;
     bool ok = true;
     float2 sw[8];
 #pragma unroll
-    for (int k = 0; k < 8; k++) sw[k] = voxel_sw<kStorage>(g, bk[k], cell_voxel(ix, iy, iz, k));
+    for (int k = 0; k < 8; k++) sw[k] = voxel_sw<kStorage>(g, cell_bucket(c, straddle, k), cell_voxel(ix, iy, iz, k));
     c.voxels += 8;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
