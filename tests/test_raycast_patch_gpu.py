@@ -1,0 +1,44 @@
+"""Ray-to-lane mappings of the raycasts: which warp and lane marches a pixel
+never shows in its result."""
+import numpy as np
+import pytest
+import torch
+
+import synth
+from superscanner_gb300 import GPUVoxelGrid
+from superscanner_gb300.pipeline import raycast_maps
+
+pytestmark = pytest.mark.gpu
+
+
+def small_grid(rows, cols, storage):
+    f = 0.8 * cols
+    intr = (f, f, cols / 2 - 0.5, rows / 2 - 0.5)
+    sc = synth.Scene(2, 31)
+    P = sc.trajectory(3, 5)
+    depth, _ = sc.render(P, rows, cols, intr, noise=True, noise_seed=3, color=False)
+    g = GPUVoxelGrid(int(1e9), 0.04, 0.01, rows, cols, storage=storage, with_color=False, hash_buckets=1 << 16,
+                     max_weight=255)
+    g.setIntrinsic(*intr)
+    for k in range(3):
+        g.integrate_fast(torch.from_numpy(np.ascontiguousarray(depth[k].view(np.int16))).cuda(),
+                         P[k].astype(np.float32))
+    return g, P[2].astype(np.float32)
+
+
+@pytest.mark.parametrize("rows,cols,launch_rows,storage", [
+    (1, 1, 8, "f32"), (3, 7, 4, "f16"), (4, 8, 4, "f32"), (5, 33, 8, "f16"), (31, 65, 16, "f32"),
+    (61, 97, 2, "f16"), (61, 97, 1, "f32"), (120, 160, 8, "f16"),
+])
+def test_maps_without_hint(rows, cols, launch_rows, storage):
+    # a hint of zeros leaves every ray its whole range, in row segments
+    g, pose = small_grid(rows, cols, storage)
+    g.set_launch_config(raycast_rows=launch_rows)
+    v, n = raycast_maps(g, pose)
+    zeros = torch.zeros((rows, cols), dtype=torch.int16, device="cuda")
+    v0, n0 = raycast_maps(g, pose, hint_depth=zeros, hint_margin=0.04)
+    g.sync()
+    assert torch.equal(v.view(torch.int32), v0.view(torch.int32))
+    assert torch.equal(n.view(torch.int32), n0.view(torch.int32))
+    if rows * cols > 1000:
+        assert (v[..., 3] > 0).float().mean() > 0.5
