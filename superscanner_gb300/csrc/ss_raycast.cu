@@ -148,14 +148,16 @@ constexpr int kHashCollisionFree = 950;
 
 template <int kStorage>
 __global__ void __launch_bounds__(256, 4) raycast_ref_kernel(GridView g, Mat34 Er, float *__restrict__ out_pcd,
-                                                          float *__restrict__ out_col, int iter_cap) {
-    // warp w of the 32 x 8 tile marches an 8 x 4 pixel patch: neighbouring rays
-    // in both directions take more similar paths than a 32-pixel row segment
-    // (0.351 vs 0.388 ms per call at 640 x 480)
+                                                          float *__restrict__ out_col, int iter_cap,
+                                                          int patch_shift) {
+    // warp w marches a patch of (1 << patch_shift) x 4 pixels, 8 x 4 or, in a small
+    // image, 4 x 4 on half its lanes: neighbouring rays in both directions take
+    // more similar paths than a 32-pixel row segment (0.351 vs 0.388 ms per call
+    // at 640 x 480)
     const int w = threadIdx.y, ln = threadIdx.x;
-    const int j = blockIdx.x * 32 + (w & 3) * 8 + (ln & 7);
-    const int i = blockIdx.y * blockDim.y + (w >> 2) * 4 + (ln >> 3);
-    if (i >= g.resi || j >= g.resj) return;
+    const int j = (((blockIdx.x << 2) + (w & 3)) << patch_shift) + (ln & ((1 << patch_shift) - 1));
+    const int i = blockIdx.y * blockDim.y + (w >> 2) * 4 + (ln >> patch_shift);
+    if (ln >= (4 << patch_shift) || i >= g.resi || j >= g.resj) return;
     const float vl = g.vl, vbl = g.vbl, dtr = g.trunc, dmax = g.d_max;
 
     const F3 np = f3normalized(get_point(g.in, i, j, 1.0f));
@@ -538,13 +540,20 @@ extern "C" ss_status ss_raycast(ss_grid *g, const float extr[16], float *ray_pcd
     for (int k = 0; k < 16; k++)
         if (!std::isfinite(extr[k])) return SS_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
-    const dim3 blk(32, 8), grid((g->p.resj + 31) / 32, (g->p.resi + 7) / 8);
+    // A warp lasts as long as its longest ray. Where full warps would be no more
+    // than four a scheduler, an image ends with its slowest warp, and warps of
+    // half the rays wait for fewer: 56 vs 61 us at 160 x 120, 80 vs 84 at
+    // 320 x 240. Beyond, the second half of the warps costs issue slots: 114 vs
+    // 92 us at 517 x 389, 173 vs 132 at 640 x 480.
+    const int64_t pixels = (int64_t)g->p.resi * g->p.resj;
+    const int shift = pixels <= (int64_t)g->num_sms * 4 * 4 * 32 ? 2 : 3;
+    const dim3 blk(32, 8), grid((g->p.resj + (4 << shift) - 1) / (4 << shift), (g->p.resi + 7) / 8);
     const Mat34 Er = mat34_from(extr);
     const int cap = g->raycast_cap > 0 ? g->raycast_cap : kRaycastIterCap;
     if (g->p.storage == SS_STORAGE_F32) {
-        raycast_ref_kernel<SS_STORAGE_F32><<<grid, blk, 0, s>>>(g->v, Er, ray_pcd, ray_color, cap);
+        raycast_ref_kernel<SS_STORAGE_F32><<<grid, blk, 0, s>>>(g->v, Er, ray_pcd, ray_color, cap, shift);
     } else {
-        raycast_ref_kernel<SS_STORAGE_F16><<<grid, blk, 0, s>>>(g->v, Er, ray_pcd, ray_color, cap);
+        raycast_ref_kernel<SS_STORAGE_F16><<<grid, blk, 0, s>>>(g->v, Er, ray_pcd, ray_color, cap, shift);
     }
     SS_LAUNCH_CHECK();
     return SS_OK;
