@@ -66,64 +66,70 @@ __device__ __forceinline__ void quad_observe_exact(const GridView &g, const uint
 // rigid E, (E p - vm) . Ez with p the pixel's point at depth d is d - q.z, the
 // distance along the camera axis (a voxel behind the camera gets d + |q.z| >
 // trunc).
-__device__ __forceinline__ bool observe_fast(const GridView &g, uint16_t depth, float qz, float &sdf) {
+// Two voxels at once, in paired instructions.
+__device__ __forceinline__ void observe_fast(const GridView &g, uint16_t depth0, uint16_t depth1, f32x2 qz, f32x2 &sdf,
+                                             bool &ok0, bool &ok1) {
     // (float)depth: 2^23 + depth, the 2^23 taken off again
-    const float d = (__uint_as_float(0x4B000000u | depth) - 8388608.f) * 1.0e-3f;
-    sdf = d - qz;
-    return d > g.rmin && fabsf(sdf) < g.trunc;
+    const f32x2 mm = f2_sub(f2_pack(__uint_as_float(0x4B000000u | depth0), __uint_as_float(0x4B000000u | depth1)),
+                            f2_pack(8388608.f, 8388608.f));
+    const f32x2 k = f2_pack(1.0e-3f, 1.0e-3f);
+    float d0, d1, s0, s1;
+    const f32x2 d = f2_mul(mm, k);
+    f2_unpack(d, d0, d1);
+    sdf = f2_sub(d, qz);
+    f2_unpack(sdf, s0, s1);
+    ok0 = ok0 && d0 > g.rmin && fabsf(s0) < g.trunc;
+    ok1 = ok1 && d1 > g.rmin && fabsf(s1) < g.trunc;
 }
 
 // The fast path's observation of a lane's four voxels r0 .. r0 + 3 (r0 even:
 // voxel (l0, m0) at vm0, then (l0 + 4, m0), (l0, m0 + 1), (l0 + 4, m0 + 1)).
 // Camera-frame points: Einv vm0 and, for the others, the transformed voxel
-// steps (4 vl along y, vl along z) added with rounded operations that are
-// never contracted. Pixels: the nearest (the reference's truncation picks the
+// steps (ystep: 4 vl along y, zstep: vl along z, from fast_steps) added with
+// rounded operations that are never contracted. Pixels: the nearest (the reference's truncation picks the
 // pixel half a pixel off the projection, which makes frame-to-model tracking
 // drift), with the half pixel of the rounding folded into the principal point
 // and the projection from an approximate reciprocal (the pixel choice only
 // needs it to ~1 ulp); the floors come from additions of 1.5 2^23 rounded down:
 // an integer below 2^22 in the sum's low bits, and for everything else
-// (infinities and NaN too) a number outside any image. Voxels 0 and 2, then 1
+// (infinities and NaN too) a number outside any image. Voxels 0 and 1, then 2
 // and 3 go through paired instructions (the same roundings); the four gathers
 // are in flight together, and no branch comes before they have arrived. The
 // per-frame fusion and the batched re-fusion share it (bit for bit the same
 // volume).
 __device__ __forceinline__ void quad_observe_fast(const GridView &g, const uint16_t *__restrict__ depth,
-                                                  const Mat34 &Einv, F3 vm0, float vl, float obs[4], bool ok[4],
-                                                  int pix[4]) {
+                                                  const Mat34 &Einv, const float ystep[3],
+                                                  const float zstep[3], F3 vm0, f32x2 obs[2], bool ok[4], int pix[4]) {
     const float ax = fmaf(vm0.x, Einv.m[0], fmaf(vm0.y, Einv.m[1], fmaf(vm0.z, Einv.m[2], Einv.m[3])));
     const float ay = fmaf(vm0.x, Einv.m[4], fmaf(vm0.y, Einv.m[5], fmaf(vm0.z, Einv.m[6], Einv.m[7])));
     const float az = fmaf(vm0.x, Einv.m[8], fmaf(vm0.y, Einv.m[9], fmaf(vm0.z, Einv.m[10], Einv.m[11])));
-    const float sy = __fmul_rn(4.f, vl);
     auto both = [](float v) { return f2_pack(v, v); };
-    f32x2 x[2], y[2], z[2];  // voxels (0, 2) and (1, 3)
-    x[0] = f2_pack(ax, __fadd_rn(ax, __fmul_rn(Einv.m[2], vl)));
-    y[0] = f2_pack(ay, __fadd_rn(ay, __fmul_rn(Einv.m[6], vl)));
-    z[0] = f2_pack(az, __fadd_rn(az, __fmul_rn(Einv.m[10], vl)));
-    x[1] = f2_add(x[0], both(__fmul_rn(Einv.m[1], sy)));
-    y[1] = f2_add(y[0], both(__fmul_rn(Einv.m[5], sy)));
-    z[1] = f2_add(z[0], both(__fmul_rn(Einv.m[9], sy)));
+    auto pair = [](float v, float ystep) { return f2_pack(v, __fadd_rn(v, ystep)); };
+    // voxels (0, 1) and (2, 3)
+    const f32x2 x[2] = {pair(ax, ystep[0]), pair(__fadd_rn(ax, zstep[0]), ystep[0])};
+    const f32x2 y[2] = {pair(ay, ystep[1]), pair(__fadd_rn(ay, zstep[1]), ystep[1])};
+    const f32x2 z[2] = {pair(az, ystep[2]), pair(__fadd_rn(az, zstep[2]), ystep[2])};
     uint16_t d[4];
-    float qz[4];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        float r[2], fi[2], fj[2];
-        f2_unpack(z[h], qz[h], qz[h + 2]);
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[0]) : "f"(qz[h]));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[1]) : "f"(qz[h + 2]));
+        float qz[2], r[2], fi[2], fj[2];
+        f2_unpack(z[h], qz[0], qz[1]);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[0]) : "f"(qz[0]));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r[1]) : "f"(qz[1]));
         const f32x2 rz = f2_pack(r[0], r[1]), big = both(12582912.f);
         f2_unpack(f2_add_down(f2_fma(f2_mul(y[h], both(g.in.fy)), rz, both(g.in.ci + 0.5f)), big), fi[0], fi[1]);
         f2_unpack(f2_add_down(f2_fma(f2_mul(x[h], both(g.in.fx)), rz, both(g.in.cj + 0.5f)), big), fj[0], fj[1]);
 #pragma unroll
         for (int u = 0; u < 2; u++) {
             const unsigned i = __float_as_uint(fi[u]) - 0x4B400000u, j = __float_as_uint(fj[u]) - 0x4B400000u;
-            pix[h + 2 * u] = (int)(i * (unsigned)g.resj + j);
-            ok[h + 2 * u] = i < (unsigned)g.resi && j < (unsigned)g.resj;
-            d[h + 2 * u] = ok[h + 2 * u] ? __ldg(depth + pix[h + 2 * u]) : (uint16_t)0;
+            const int rr = 2 * h + u;
+            pix[rr] = (int)(i * (unsigned)g.resj + j);
+            ok[rr] = i < (unsigned)g.resi && j < (unsigned)g.resj;
+            d[rr] = ok[rr] ? __ldg(depth + pix[rr]) : (uint16_t)0;
         }
     }
 #pragma unroll
-    for (int rr = 0; rr < 4; rr++) ok[rr] = observe_fast(g, d[rr], qz[rr], obs[rr]) && ok[rr];
+    for (int h = 0; h < 2; h++) observe_fast(g, d[2 * h], d[2 * h + 1], z[h], obs[h], ok[2 * h], ok[2 * h + 1]);
 }
 
 // x / y for a weight y (1 .. 2^24): x times the approximate reciprocal, as
@@ -150,6 +156,34 @@ __device__ __forceinline__ void running_average(float &s, float &w, float obs, f
             w = 0.f;
             s = 0.f;
         }
+    }
+}
+
+// The fast update of two voxels at once (the same roundings), weights capped.
+template <bool kDeint, int kStorage>
+__device__ __forceinline__ void running_average_pair(float &s0, float &s1, float &w0, float &w1, f32x2 obs, bool ok0,
+                                                     bool ok1, float cap, float trunc, float inv_trunc) {
+    const f32x2 w = f2_pack(w0, w1), one = f2_pack(1.f, 1.f);
+    const f32x2 v = kDeint ? f2_sub(w, one) : f2_add(w, one);
+    float v0, v1, r0, r1, a0, a1;
+    f2_unpack(v, v0, v1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(v0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(v1));
+    const f32x2 a = f2_mul(f2_fma(f2_pack(s0, s1), w, kDeint ? f2_neg(obs) : obs), f2_pack(r0, r1));
+    if (kStorage == SS_STORAGE_F16) {  // the value a sequential call would have stored
+        f2_unpack(f2_mul(a, f2_pack(inv_trunc, inv_trunc)), a0, a1);
+        const float2 h = __half22float2(__floats2half2_rn(a0, a1));
+        f2_unpack(f2_mul(f2_pack(h.x, h.y), f2_pack(trunc, trunc)), a0, a1);
+    } else {
+        f2_unpack(a, a0, a1);
+    }
+    if (ok0) {
+        s0 = kDeint && v0 == 0.f ? 0.f : a0;
+        w0 = kDeint ? v0 : fminf(v0, cap);
+    }
+    if (ok1) {
+        s1 = kDeint && v1 == 0.f ? 0.f : a1;
+        w1 = kDeint ? v1 : fminf(v1, cap);
     }
 }
 

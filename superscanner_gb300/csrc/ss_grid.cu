@@ -227,7 +227,14 @@ __global__ void __launch_bounds__(256, kColor ? 4 : kExact ? 5 : 8) fuse_kernel(
         if (kExact)
             quad_observe_exact(g, depth, E, Einv, Ez, vm0, F3{pzx, pzy, pzz}, l0, r0, obs4, ok, pix4);
         else
-            quad_observe_fast(g, depth, Einv, vm0, g.vl, obs4, ok, pix4);
+ {
+            float ystep[3], zstep[3];
+            fast_steps(Einv, g.vl, ystep, zstep);
+            f32x2 o[2];
+            quad_observe_fast(g, depth, Einv, ystep, zstep, vm0, o, ok, pix4);
+            f2_unpack(o[0], obs4[0], obs4[1]);
+            f2_unpack(o[1], obs4[2], obs4[3]);
+        }
         // the colours of the voxels that change, and their pixels', all in flight together
         float col[4][3];
         uint8_t seen[4][3];
@@ -631,8 +638,7 @@ ss_status ss_grid_destroy(ss_grid *g) {
     cudaFree(g->phase_mask);
     cudaFree(g->mesh_count);
     cudaFree(g->t_hit);
-    cudaFree(g->batch_poses);
-    cudaFree((void *)g->batch_depths);
+    cudaFree(g->batch_phases);
     delete g;
     return SS_OK;
 }

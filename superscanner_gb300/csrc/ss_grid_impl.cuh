@@ -21,8 +21,7 @@ struct ss_grid {
     int num_sms = 0;
     // batched re-fusion scratch, allocated on the first ss_refuse_batch call
     uint32_t *phase_mask = nullptr;        // [buckets][kMaxPhases / 32]
-    ss::FramePose *batch_poses = nullptr;  // [kMaxPhases]
-    const uint16_t **batch_depths = nullptr;  // [kMaxPhases / 2] device pointers
+    ss::RefusePhase *batch_phases = nullptr;  // [kMaxPhases]
     unsigned long long *mesh_count = nullptr;  // triangle and bucket counters of mesh extraction (first call)
     float *t_hit = nullptr;                // [resi][resj] hit depths of the differentiable raycast (first call)
     // launch collect, fuse and raycast as programmatic dependents of the kernel

@@ -74,6 +74,22 @@ struct __align__(16) FramePose {  // 16-byte aligned: a kernel loads E or Einv a
     float pad;
 };
 
+// One phase of a batched re-fusion: its pose, the voxel steps of the fast
+// observation in its camera (4 vl along y, vl along z) and its depth image.
+struct __align__(16) RefusePhase {
+    FramePose pose;
+    float ystep[3], zstep[3];
+    const uint16_t *depth;
+};
+
+// A voxel step of 4 vl along y and one of vl along z, in the camera.
+__host__ __device__ __forceinline__ void fast_steps(const Mat34 &Einv, float vl, float ystep[3], float zstep[3]) {
+    for (int a = 0; a < 3; a++) {
+        ystep[a] = Einv.m[4 * a + 1] * (4.f * vl);
+        zstep[a] = Einv.m[4 * a + 2] * vl;
+    }
+}
+
 __device__ __forceinline__ void load_pose(const FramePose *p, Mat34 &E, Mat34 &Einv, float &ezx, float &ezy,
                                           float &ezz) {
 #pragma unroll
@@ -391,6 +407,11 @@ __device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
 }
 __device__ __forceinline__ void f2_unpack(f32x2 v, float &lo, float &hi) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 f2_neg(f32x2 v) {
+    float lo, hi;
+    f2_unpack(v, lo, hi);
+    return f2_pack(-lo, -hi);
 }
 __device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
     f32x2 r;
