@@ -181,9 +181,9 @@ __global__ void __launch_bounds__(256, 8) collect_kernel(GridView g, const uint1
 // capped at 32 (8 CTAs, 64 warps per SM: the kernel waits on dependent loads;
 // 16.0 -> 12.7 us for a frame of 1280 x 720). The reference's arithmetic holds
 // more values between the gathers and the updates: 48 registers (5 CTAs; FP16
-// 517 x 389 20 -> 17 us, 19 us at 32), and with colour, whose twelve plane
+// 517 x 389 20 -> 17 us, 19 us at 32; now 15.4), and with colour, whose twelve plane
 // values and pixel bytes are loaded together too, 64 (4 CTAs; FP32 640 x 480 50
-// -> 36 us; 40 at 48 and 39 at 77).
+// -> 36 us, 40 at 48 and 39 at 77; now 32).
 template <int kStorage, bool kColor, bool kDeint, bool kExact>
 __global__ void __launch_bounds__(256, kColor ? 4 : kExact ? 5 : 8) fuse_kernel(GridView g, const uint16_t *__restrict__ depth,
                                                    const uint8_t *__restrict__ rgb, Mat34 E, Mat34 Einv, F3 Ez,

@@ -398,7 +398,9 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Packed pairs of floats (a 64-bit register pair: lane 0 in the low half)
 // and the paired FP32 instructions of this architecture: each half rounded to
 // nearest as the scalar instruction would, so one instruction does the arithmetic of two
-// independent values.
+// independent values. The assembler contracts a paired product and sum into a
+// fused one, .rn or not; where the product's rounding is part of the result, it
+// is written as a fused one with an addend of -0 that only the kernel knows.
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 f2_pack(float lo, float hi) {
     f32x2 r;
@@ -438,6 +440,15 @@ __device__ __forceinline__ f32x2 f2_add_down(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
+}
+
+// depth_m of two depths.
+__device__ __forceinline__ f32x2 depth_m_pair(uint16_t d0, uint16_t d1) {
+    auto both = [](float v) { return f2_pack(v, v); };
+    // (float)d: 2^23 + d, the 2^23 taken off again
+    const f32x2 a = f2_sub(f2_pack(__uint_as_float(0x4B000000u | d0), __uint_as_float(0x4B000000u | d1)), both(8388608.f));
+    const f32x2 y = both(1.0e-3f), q0 = f2_mul(a, y);
+    return f2_fma(f2_fma(q0, both(-1000.f), a), y, q0);
 }
 
 // Exact cross-CTA sums in fixed point (resolution 2^-48): a CTA's float

@@ -102,8 +102,11 @@ __global__ void __launch_bounds__(256, 8) refuse_collect_kernel(GridView g, cons
 // four observations come first, without branches (ss_fuse.cuh), and a row of
 // voxels none of which is seen skips its update: 100 keyframes of 640 x 480
 // 1.20 -> 0.89 ms. Observations and updates in pairs of voxels, with the
-// phases' voxel steps laid out with their poses: 0.89 -> 0.84 ms. The next phase's gathers ahead of this phase's update were
-// slower (24 % at 48 registers, 4 % at 40).
+// phases' voxel steps laid out with their poses: 0.89 -> 0.84 ms. The next
+// phase's gathers ahead of this phase's update were slower (24 % at 48
+// registers, 4 % at 40), as were gathers from a copy in 8 x 8 pixel lines (0.95
+// ms) and phases left out by the depth extremes of their pixels (1.07 ms: a
+// sixth of the unobserved could be told from them).
 template <int kStorage, bool kExact>
 __global__ void __launch_bounds__(256) refuse_apply_kernel(GridView g, const RefusePhase *__restrict__ phases,
                                                            const uint32_t *__restrict__ phase_mask) {

@@ -104,8 +104,9 @@ def test_index_shortcuts_give_the_reference_rules():
 
 
 def test_projected_pixel_shortcut_gives_the_reference_cast():
-    """project_axis_fast (ss_fuse.cuh): wherever its test is decisive, for any reciprocal within 1 ulp of 1 / z, the
-    truncated coordinate is that of the reference's IEEE quotient; undecided only near pixel edges."""
+    """project_axis_pair (ss_fuse.cuh): wherever its test is decisive, for any reciprocal within 1 ulp of 1 / z, its
+    pixel is the truncated coordinate of the reference's IEEE quotient, or both lie outside the image; undecided only
+    near pixel edges."""
     rng = np.random.default_rng(5)
     for f, c, n in ((525.0, 319.5, 640), (131.25, 60.5, 120), (2100.0, 1279.5, 4096), (60.0, -3.0, 64)):
         f, c = F(f), F(c)
@@ -118,6 +119,10 @@ def test_projected_pixel_shortcut_gives_the_reference_cast():
         y = (1.0 / z.astype(np.float64)).astype(F)
         for rz in (y, np.nextafter(y, F(np.inf)), np.nextafter(y, F(-np.inf))):
             a = (pf.astype(np.float64) * rz.astype(np.float64) + float(c)).astype(F)
-            sure = np.abs(a - np.rint(a)) > F(4.0e-7) * (np.abs(a) + np.abs(c))
-            assert np.array_equal(np.trunc(a).astype(np.int64)[sure], want[sure])
+            fl = np.floor(a)
+            decide = F(0.5) - F(4.0e-7) * (F(n + 2) + np.abs(c))
+            sure = np.abs((a - fl) - F(0.5)) < decide
+            got = fl.astype(np.int64) + (fl < 0)
+            outside = ((got < 0) | (got >= n)) & ((want < 0) | (want >= n))
+            assert (np.where(outside, want, got) == want)[sure].all()
             assert sure[1::3].mean() > 0.98
