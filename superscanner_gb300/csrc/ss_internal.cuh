@@ -383,6 +383,10 @@ __device__ __forceinline__ bool super_occupied(const GridView &g, int sx, int sy
     return false;
 }
 
+// floor(u) for |u| < 2^22, from an addition of 1.5 2^23 rounded down; beyond,
+// a number of magnitude 2^22 or more.
+__device__ __forceinline__ int floor_int(float u) { return __float_as_int(__fadd_rd(u, 12582912.f)) - 0x4B400000; }
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 // Programmatic dependent launch. A kernel launched with the programmatic

@@ -407,7 +407,7 @@ extern "C" int ss_debug_raycast_timing(unsigned long long *out, int reset) {
     } while (0)
 #endif
 
-template <int kStorage>
+template <int kStorage, bool kHint>
 __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 T, const FramePose *__restrict__ pose,
                                                            int max_steps, float t_min, float t_max,
                                                            float4 *__restrict__ vmap, float4 *__restrict__ nmap,
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 
     // its hint from. Without one the rays march all the way, where an 8 x 4 patch
     // keeps together better than a row (240 vs 258 us at 640 x 480, 418 vs 479 us
     // at 1280 x 720; it takes a CTA of a multiple of four rows).
-    const bool patch = !hint && (blockDim.y & 3) == 0;
+    const bool patch = !kHint && (blockDim.y & 3) == 0;
     const int j = blockIdx.x * 32 + (patch ? (threadIdx.y & 3) * 8 + (threadIdx.x & 7) : threadIdx.x);
     const int i = blockIdx.y * blockDim.y + (patch ? (threadIdx.y >> 2) * 4 + (threadIdx.x >> 3) : threadIdx.y);
     const bool inside = i < g.resi && j < g.resj;
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 
     // that is missing (dropout), the smaller depth of the nearest pixels with
     // depth to its left and right within this warp's 32-pixel row segment.
     unsigned hint_mm = 0;
-    if (hint) {
+    if (kHint) {
         const unsigned full = 0xffffffffu;
         const int lane = threadIdx.x & 31;
         const unsigned own = inside ? (unsigned)__ldg(hint + (size_t)i * g.resj + j) : 0u;
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(512, 2) raycast_maps_kernel(GridView g, Mat34 
 
     float t = t_min;
     const float t_hint = (float)hint_mm * 1e-3f - hint_margin;
-    if (hint && t_hint > t_min) {
+    if (kHint && t_hint > t_min) {
         // seek from the hint d within [d - margin, d + margin]
         hit = ray_search<kStorage>(g, ox, oy, oz, dx, dy, dz, inv_len, kRaySeek, t_hint + hint_margin, t_hint,
                                    fminf(t_max, t_hint + 2.f * hint_margin), max_steps, steps, t, cache);
@@ -520,12 +520,21 @@ ss_status launch_raycast_maps(ss_grid *g, const Mat34 &T, const FramePose *dpose
                               const uint16_t *hint, float hint_margin, Counters *end) {
     const int rr = g->lc.raycast_rows;
     const dim3 blk(32, rr), grid((g->p.resj + 31) / 32, (g->p.resi + rr - 1) / rr);
-    if (g->p.storage == SS_STORAGE_F32)
-        SS_CUDA_TRY(launch_kernel(raycast_maps_kernel<SS_STORAGE_F32>, grid, blk, 0, s, g->pdl, g->v, T, dpose, max_steps,
-                                  t_min, t_max, vmap, nmap, counters, hint, hint_margin, end));
-    else
-        SS_CUDA_TRY(launch_kernel(raycast_maps_kernel<SS_STORAGE_F16>, grid, blk, 0, s, g->pdl, g->v, T, dpose, max_steps,
-                                  t_min, t_max, vmap, nmap, counters, hint, hint_margin, end));
+#define SS_RM(ST, HINT)                                                                                             \
+    SS_CUDA_TRY(launch_kernel(raycast_maps_kernel<ST, HINT>, grid, blk, 0, s, g->pdl, g->v, T, dpose, max_steps, t_min, \
+                              t_max, vmap, nmap, counters, hint, hint_margin, end))
+    if (g->p.storage == SS_STORAGE_F32) {
+        if (hint)
+            SS_RM(SS_STORAGE_F32, true);
+        else
+            SS_RM(SS_STORAGE_F32, false);
+    } else {
+        if (hint)
+            SS_RM(SS_STORAGE_F16, true);
+        else
+            SS_RM(SS_STORAGE_F16, false);
+    }
+#undef SS_RM
     return SS_OK;
 }
 

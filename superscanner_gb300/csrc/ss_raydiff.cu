@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(32 * kMarchWarps) raymarch_kernel(GridView g, 
         BlockCache cache(buckets, threadIdx.x, 32 * kMarchWarps);
         int steps = 0;
         float t = t_min;
-        const bool hit = march<kStorage>(g, T.m[3], T.m[7], T.m[11], dx, dy, dz, inv_len, t_min, t_max, max_steps,
-                                         steps, t, cache);
+        const bool hit = march<kStorage, 2>(g, T.m[3], T.m[7], T.m[11], dx, dy, dz, inv_len, t_min, t_max, max_steps,
+                                            steps, t, cache);
         t_hit[(size_t)i * g.resj + j] = hit ? t : __int_as_float(0x7fc00000);
     }
 }

@@ -43,6 +43,13 @@ __device__ __forceinline__ float2 voxel_sw(const GridView &g, int bucket, int v)
     }
 }
 
+// Whether the voxel is observed (its weight positive).
+template <int kStorage>
+__device__ __forceinline__ bool voxel_seen(const GridView &g, int bucket, int v) {
+    const size_t vi = (size_t)bucket * kBlockVoxels + v;
+    return kStorage == SS_STORAGE_F32 ? __ldg(&g.vox32[vi].y) > 0.f : __ldg(g.vox16 + vi) > 0xFFFFu;
+}
+
 __device__ __forceinline__ int cached_lookup(const GridView &g, BlockCache &c, int bx, int by, int bz) {
     if (bx == c.x && by == c.y && bz == c.z) return c.bucket;
     c.x = bx;
@@ -196,7 +203,14 @@ constexpr int kRaySeek = 1;     // search near a depth hint t0 within [t_lo, t_h
 // Forward marching ends at t_hi. Every sample or skip counts as one step. A
 // bracket is refined by two regula-falsi steps, then the secant root is the
 // hit (t).
-template <int kStorage>
+// Four of five samples of a forward march from the camera are invalid, in runs
+// of one-voxel steps. With kAhead a turn first tells, each by one voxel, which
+// of the next kAhead points are: a cell's corner nearest to the camera is the
+// last to be observed. Only where that corner and the point lie in the block
+// of this turn; the other points are sampled as ever. Two points: 200 -> 191
+// us (640 x 480, 4 mm), 169 -> 158 (517 x 389, 6 mm); one 170, three 162, six
+// 195.
+template <int kStorage, int kAhead = 0>
 __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy, float oz, float dx, float dy,
                                            float dz, float inv_len, int mode, float t0, float t_lo, float t_hi,
                                            int max_steps, int &steps, float &t, BlockCache &cache) {
@@ -215,7 +229,7 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
     // their warp only behind the loop
     bool go = steps < max_steps && (mode != kRayForward || t < t_hi);
     while (go) {
-        const float px = fmaf(t, dx, ox), py = fmaf(t, dy, oy), pz = fmaf(t, dz, oz);
+        float px = fmaf(t, dx, ox), py = fmaf(t, dy, oy), pz = fmaf(t, dz, oz);
         steps++;
         bool skip = false;
         if (mode == kRayForward) {
@@ -243,6 +257,42 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
                 prev_valid = false;
             }
         }
+        if (kAhead > 0 && !skip && mode == kRayForward) {
+            float at[kAhead + 1];  // t after so many invalid samples
+            bool unseen[kAhead + 1];
+            at[0] = t;
+            const int bx = floor_int(px * inv_vbl), by = floor_int(py * inv_vbl), bz = floor_int(pz * inv_vbl);
+            const int nx = dx > 0.f ? 0 : 1, ny = dy > 0.f ? 0 : 1, nz = dz > 0.f ? 0 : 1;  // the nearest corner
+#pragma unroll
+            for (int m = 0; m < kAhead; m++) {
+                const float x = fmaf(at[m], dx, ox), y = fmaf(at[m], dy, oy), z = fmaf(at[m], dz, oz);
+                const int vx = floor_int(fmaf(x, inv_vl, -0.5f)) + nx, vy = floor_int(fmaf(y, inv_vl, -0.5f)) + ny,
+                          vz = floor_int(fmaf(z, inv_vl, -0.5f)) + nz;
+                unseen[m] = at[m] < t_hi && (vx >> 3) == bx && (vy >> 3) == by && (vz >> 3) == bz &&
+                            floor_int(x * inv_vbl) == bx && floor_int(y * inv_vbl) == by && floor_int(z * inv_vbl) == bz;
+                if (unseen[m])  // cache.bucket: the block's, looked up above
+                    unseen[m] = !voxel_seen<kStorage>(g, cache.bucket, (vx & 7) + 8 * (vy & 7) + 64 * (vz & 7));
+                at[m + 1] = fmaf(vl, inv_len, at[m]);
+            }
+            steps--;  // counted point by point from here
+            bool run = true;
+#pragma unroll
+            for (int m = 0; m < kAhead; m++) {
+                run = run && unseen[m] && steps < max_steps;
+                if (run) {
+                    steps++;
+                    t = at[m + 1];
+                    prev_valid = false;
+                }
+            }
+            skip = run || !(steps < max_steps && t < t_hi);
+            if (!skip) {
+                px = fmaf(t, dx, ox), py = fmaf(t, dy, oy), pz = fmaf(t, dz, oz);
+                // a point past the block takes a turn of its own
+                skip = !(floor_int(px * inv_vbl) == bx && floor_int(py * inv_vbl) == by && floor_int(pz * inv_vbl) == bz);
+                if (!skip) steps++;
+            }
+        }
         bool end = false;
         if (!skip) {
             const TriSample sm = trilinear<kStorage, false>(g, px, py, pz, inv_vl, cache);
@@ -251,7 +301,7 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
             if (mode == kRayForward) {
                 if (!sm.valid) {
                     prev_valid = false;
-                    t += vl * inv_len;
+                    t = fmaf(vl, inv_len, t);
                 } else if (neg) {
                     found = prev_valid && f_prev > 0.f;  // else a back face
                     ta = t_prev;
@@ -303,12 +353,12 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
 }
 
 // One forward ray march from t0 to t_max; returns true on a zero crossing (t = hit depth).
-template <int kStorage>
+template <int kStorage, int kAhead = 0>
 __device__ __forceinline__ bool march(const GridView &g, float ox, float oy, float oz, float dx, float dy, float dz,
                                       float inv_len, float t0, float t_max, int max_steps, int &steps, float &t,
                                       BlockCache &cache) {
-    return ray_search<kStorage>(g, ox, oy, oz, dx, dy, dz, inv_len, kRayForward, t0, t0, t_max, max_steps, steps, t,
-                                cache);
+    return ray_search<kStorage, kAhead>(g, ox, oy, oz, dx, dy, dz, inv_len, kRayForward, t0, t0, t_max, max_steps, steps,
+                                        t, cache);
 }
 
 }  // namespace ss

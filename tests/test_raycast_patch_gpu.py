@@ -1,5 +1,5 @@
-"""Ray-to-lane mappings of the raycasts: which warp and lane marches a pixel
-never shows in its result."""
+"""Forms of the raycasts' marches: which warp and lane marches a pixel, and how
+many of its samples a turn tells, never shows in its result."""
 import numpy as np
 import pytest
 import torch
@@ -8,6 +8,7 @@ import oracle
 import synth
 from superscanner_gb300 import GPUVoxelGrid
 from superscanner_gb300.pipeline import raycast_maps
+from superscanner_gb300.raydiff import raycast_loss
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,23 @@ def test_reference_raycast(rows, cols):
     assert np.all(got == want, axis=-1).mean() >= 0.999
     if rows * cols > 1000:
         assert (want[..., 2] != 0).mean() > 0.9
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("max_steps", [1, 2, 7, 18, 19, 20, 21, 33, 128])
+def test_march_ahead(storage, max_steps):
+    # the differentiable raycast's march tells several invalid samples a turn; it
+    # ends after the same steps as the view's, which takes them one by one, and
+    # gives a ray the hit of a longer march or none
+    g, pose = small_grid(61, 97, storage)
+    obs = torch.zeros((61, 97), dtype=torch.int16, device="cuda")
+    full, depth = torch.zeros((61, 97), device="cuda"), torch.zeros((61, 97), device="cuda")
+    raycast_loss(g, pose, obs, max_steps=400, depth_out=full)
+    raycast_loss(g, pose, obs, max_steps=max_steps, depth_out=depth)
+    t_min, t_max = float(np.float32(0.2)), float(np.float32(10.0))  # the grid's depth range
+    v, _ = raycast_maps(g, pose, max_steps=max_steps, t_min=t_min, t_max=t_max)
+    g.sync()
+    hit = (v[..., 3] > 0) & (full > 0)
+    assert torch.equal(depth, torch.where(hit, full, torch.zeros_like(full)))
+    if max_steps == 128:
+        assert hit.float().mean() > 0.5
