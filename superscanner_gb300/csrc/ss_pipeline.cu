@@ -346,7 +346,9 @@ ss_status ss_pipeline_frame(ss_pipeline *P, const uint16_t *depth, int32_t track
         }
         SS_CUDA_TRY(cudaGraphLaunch(P->exec[b], s));
     } else {
+        g->pdl = !P->profile;  // as in the graph; the profile's events sit between the kernels
         st = enqueue_frame(P, in, s, P->profile, P->test_wait_polls);
+        g->pdl = false;
         P->test_wait_polls = 0;
         if (st != SS_OK) return st;
     }

@@ -107,6 +107,7 @@ __global__ void track_begin_kernel(TrackState *st) {
 }
 
 __global__ void pose_prep_kernel(TrackState *st) {
+    pdl_wait();  // the last iteration, where one came before
     if (threadIdx.x == 0) write_frame_pose(st->T, &st->pose);
 }
 
@@ -142,6 +143,7 @@ __device__ __forceinline__ float det2(float a, float b, float c, float d) { retu
 // a group adds at most kTrackGroup - 1 roundings).
 constexpr int kTrackGroup = 4;
 
+template <int kGroup>
 __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ depth, int rows, int cols, Intr in,
                                                  const float4 *__restrict__ vmap, const float4 *__restrict__ nmap,
                                                  const float *T, const float *Pi, int level, float dist2, float rmin,
@@ -150,22 +152,22 @@ __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ de
     const int npix = lr * lc;
     const float rfx = 1.f / in.fx, rfy = 1.f / in.fy;
     PixelWalk at(tid, nthreads, lc);
-    for (int base = tid; base < npix; base += kTrackGroup * nthreads) {
-        float d[kTrackGroup];
-        int pi[kTrackGroup], pj[kTrackGroup];
+    for (int base = tid; base < npix; base += kGroup * nthreads) {
+        float d[kGroup];
+        int pi[kGroup], pj[kGroup];
 #pragma unroll
-        for (int g = 0; g < kTrackGroup; g++) {
+        for (int g = 0; g < kGroup; g++) {
             const int p = base + g * nthreads;
             pi[g] = at.i << level;
             pj[g] = at.j << level;
             at.next();
             d[g] = p < npix ? (float)__ldg(depth + (size_t)pi[g] * cols + pj[g]) * 1e-3f : 0.f;
         }
-        float wv[kTrackGroup][3];
-        float4 n[kTrackGroup], v[kTrackGroup];
-        bool ok[kTrackGroup];
+        float wv[kGroup][3];
+        float4 n[kGroup], v[kGroup];
+        bool ok[kGroup];
 #pragma unroll
-        for (int g = 0; g < kTrackGroup; g++) {
+        for (int g = 0; g < kGroup; g++) {
             const float dd = d[g];
             const float cx = ((float)pj[g] - in.cj) * rfx * dd, cy = ((float)pi[g] - in.ci) * rfy * dd;
             const float wx = fmaf(T[0], cx, fmaf(T[1], cy, fmaf(T[2], dd, T[3])));
@@ -195,7 +197,7 @@ __device__ __forceinline__ void track_accumulate(const uint16_t *__restrict__ de
         for (int q = 0; q < kTrackSums - 1; q++) t[q] = 0.f;
         bool any = false;
 #pragma unroll
-        for (int g = 0; g < kTrackGroup; g++) {
+        for (int g = 0; g < kGroup; g++) {
             if (!ok[g]) continue;
             const float4 nn = n[g], vv = v[g];
             if (nn.x == 0.f && nn.y == 0.f && nn.z == 0.f) continue;
@@ -605,11 +607,22 @@ __device__ __forceinline__ void track_slots_to_pairs(const float2 *__restrict__ 
 // Value of a (sum, compensation) pair.
 __device__ __forceinline__ float pair_value(float2 p) { return p.x - p.y; }
 
-__global__ void __launch_bounds__(256) track_iter_kernel(const uint16_t *__restrict__ depth, int rows, int cols,
-                                                         Intr in, const float4 *__restrict__ vmap,
-                                                         const float4 *__restrict__ nmap, TrackState *st,
-                                                         float2 *__restrict__ partials, int level, float dist2,
-                                                         float rmin, float dmax) {
+// One iteration of the launch-by-launch tracker: bound by latency (its launch,
+// one pixel group, the last CTA's sums and solve) and, at fine levels, by the
+// pixels. A programmatic dependent of the iteration before; no CTAs without
+// pixels (launch_track); groups of one where every pixel has a thread; 128
+// registers, so that all of L.ctas (two per SM) are resident: at 165 they ran in two
+// waves. A frame of 160 x 120 270 -> 161 us, 640 x 480 376 -> 276, 1280 x 720
+// 532 -> 407 (the CTAs 59, 12 and 6 us of it, the dependent launches 35, 34
+// and 30, two CTAs per SM 0, 42 and 75).
+template <int kGroup>
+__global__ void __launch_bounds__(256, 2) track_iter_kernel(const uint16_t *__restrict__ depth, int rows, int cols,
+                                                            Intr in, const float4 *__restrict__ vmap,
+                                                            const float4 *__restrict__ nmap, TrackState *st,
+                                                            float2 *__restrict__ partials, int level, float dist2,
+                                                            float rmin, float dmax) {
+    pdl_wait();     // the iteration before (and, through it, all that this reads)
+    pdl_trigger();  // the next iteration may launch
     if (*(volatile int *)&st->converged_level == level) return;
     __shared__ float2 red[8][kTrackSums];
     __shared__ bool last;
@@ -623,8 +636,8 @@ __global__ void __launch_bounds__(256) track_iter_kernel(const uint16_t *__restr
     float s[kTrackSums], c[kTrackSums];
 #pragma unroll
     for (int k = 0; k < kTrackSums; k++) s[k] = c[k] = 0.f;
-    track_accumulate(depth, rows, cols, in, vmap, nmap, T, Pi, level, dist2, rmin, dmax,
-                     blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, s, c);
+    track_accumulate<kGroup>(depth, rows, cols, in, vmap, nmap, T, Pi, level, dist2, rmin, dmax,
+                             blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, s, c);
     track_cta_to_slots(s, c, red, partials);
     __threadfence();
     __syncthreads();
@@ -769,8 +782,8 @@ __global__ void __launch_bounds__(256) track_frame_kernel(const uint16_t *__rest
                 else
                     track_accumulate_cam<kTrackGroup>(cam, m_count, rows, cols, in, vmap, nmap, T, P, dist2, s, c);
             else
-                track_accumulate(depth, rows, cols, in, vmap, nmap, T, P, level, dist2, L.rmin, L.dmax, tid, nthreads,
-                                 s, c);
+                track_accumulate<kTrackGroup>(depth, rows, cols, in, vmap, nmap, T, P, level, dist2, L.rmin, L.dmax,
+                                              tid, nthreads, s, c);
             SS_TT(barriers, 1);
             unsigned long long *buf = acc + (size_t)abuf * kTrackAccBufWords;
             track_cta_to_acc(s, c, red, buf);
@@ -904,14 +917,19 @@ ss_status launch_track(const TrackLaunch &L, cudaStream_t s) {
     track_begin_kernel<<<1, 32, 0, s>>>(L.state);
     SS_LAUNCH_CHECK();
     for (int level = L.levels - 1; level >= 0; level--) {
+        // no more CTAs than give every pixel of the level a thread of its own: the
+        // others would only add zeros, and the last CTA reads every CTA's sums. A
+        // group's other places would stay empty then, so it has one.
+        const int lr = (L.rows + (1 << level) - 1) >> level, lc = (L.cols + (1 << level) - 1) >> level;
+        const int ctas = std::min(L.ctas, (lr * lc + 255) / 256);
+        auto kernel = lr * lc <= 256 * ctas ? track_iter_kernel<1> : track_iter_kernel<kTrackGroup>;
         for (int it = 0; it < L.iters[level]; it++) {
-            track_iter_kernel<<<L.ctas, 256, 0, s>>>(L.depth, L.rows, L.cols, L.in, L.vmap, L.nmap, L.state, L.partials,
-                                                     level, L.dist[level] * L.dist[level], L.rmin, L.dmax);
-            SS_LAUNCH_CHECK();
+            SS_CUDA_TRY(launch_kernel(kernel, dim3(ctas), dim3(256), 0, s, true, L.depth, L.rows, L.cols, L.in,
+                                      L.vmap, L.nmap, L.state, L.partials, level, L.dist[level] * L.dist[level], L.rmin,
+                                      L.dmax));
         }
     }
-    pose_prep_kernel<<<1, 32, 0, s>>>(L.state);
-    SS_LAUNCH_CHECK();
+    SS_CUDA_TRY(launch_kernel(pose_prep_kernel, dim3(1), dim3(32), 0, s, true, L.state));
     return SS_OK;
 }
 
