@@ -538,8 +538,10 @@ struct IcpBest {
 // vertical pixel pair's windows share nine of their rows): a half row's taps
 // are loaded once, before their comparisons, and each tap's distances
 // (kokkosICP.cpp:101-102) to both source points are evaluated together
-// (packed pairs of the two points' coordinates px, py, pz), with the
-// reference's roundings in its order.
+// (packed pairs of the two points' coordinates px, py, pz). The products of the
+// distance are fused into its sum, in the order that the assembler contracted
+// them in when they were written apart (as a sum of rounded products it takes
+// two instructions more a tap).
 __device__ __forceinline__ void icp_scan_row(const float4 *sA, const float *u, float v, int row, f32x2 px, f32x2 py,
                                              f32x2 pz, bool ua, IcpBest &ba, bool ub, IcpBest &bb) {
 #pragma unroll
@@ -555,8 +557,8 @@ __device__ __forceinline__ void icp_scan_row(const float4 *sA, const float *u, f
             const f32x2 dx = f2_sub(f2_pack(y.x, y.x), px), dy = f2_sub(f2_pack(y.y, y.y), py),
                         dz = f2_sub(f2_pack(y.z, y.z), pz);
             float da, db;
-            f2_unpack(f2_add(f2_add(f2_mul(dx, f2_pack(a[dl].y, a[dl].y)), f2_mul(dy, f2_pack(a[dl].z, a[dl].z))),
-                             f2_mul(dz, f2_pack(a[dl].w, a[dl].w))),
+            f2_unpack(f2_fma(dz, f2_pack(a[dl].w, a[dl].w),
+                             f2_fma(dx, f2_pack(a[dl].y, a[dl].y), f2_mul(dy, f2_pack(a[dl].z, a[dl].z)))),
                       da, db);
             if (ua) ba.take(odd, fabsf(da), idx);
             if (ub) bb.take(odd, fabsf(db), idx);
@@ -587,7 +589,8 @@ __device__ __forceinline__ int icp_coop_plane(const float4 *sA, const float *su,
                 const int r = r0 + t / (2 * kIcpSearch), c = c0 + t % (2 * kIcpSearch);
                 const float4 a = sA[r * sw + c];
                 const F3 y = icp_tap_point(a, su[c], su[kIcpEdge + r]);
-                const float dist = fabsf(f3dot(f3sub(y, p), F3{a.y, a.z, a.w}));
+                const F3 d = f3sub(y, p);  // the distance as icp_scan_row rounds it
+                const float dist = fabsf(fmaf(d.z, a.w, fmaf(d.x, a.y, __fmul_rn(d.y, a.z))));
                 if (dist < smallest) {
                     smallest = dist;
                     tap = t;
