@@ -287,6 +287,27 @@ __device__ __forceinline__ int table_find(const GridView &g, unsigned long long 
     return -1;
 }
 
+// table_find with its probe loop out of line behind the first probe, which
+// decides nearly always: inlined, the loop keeps a march's lanes apart (and its
+// registers, where they are capped, are worth more: the views keep table_find).
+static __device__ __noinline__ int table_find_on(const unsigned long long *keys, uint32_t mask, unsigned long long key) {
+    uint32_t b = home_bucket(key, mask);
+    for (uint32_t probe = 0; probe <= mask; probe++) {
+        const unsigned long long k = __ldg(keys + b);
+        if (k == key) return (int)b;
+        if (k == kEmptyKey) return -1;
+        b = (b + 1) & mask;
+    }
+    return -1;
+}
+__device__ __forceinline__ int table_find_split(const GridView &g, unsigned long long key) {
+    const uint32_t home = home_bucket(key, g.mask);
+    const unsigned long long k0 = __ldg(g.keys + home);
+    int b = k0 == key ? (int)home : -1;
+    if (k0 != key && k0 != kEmptyKey) b = table_find_on(g.keys, g.mask, key);
+    return b;
+}
+
 // Lock-free find-or-insert (UnorderedMap::find + insert,
 // GPUVoxelGrid.cpp:493-499). Returns the bucket, or -1 with kStTableFull set.
 // Inserts claim the first tombstone or the terminating empty bucket of the
@@ -381,6 +402,25 @@ __device__ __forceinline__ bool super_occupied(const GridView &g, int sx, int sy
         b = (b + 1) & g.sbmask;
     }
     return false;
+}
+
+// super_occupied with its probe loop out of line, as table_find_split.
+static __device__ __noinline__ bool super_occupied_on(const unsigned long long *keys, uint32_t mask,
+                                                      unsigned long long key) {
+    uint32_t b = super_home(key, mask);
+    for (uint32_t probe = 0; probe <= mask; probe++) {
+        const unsigned long long k = __ldg(keys + b);
+        if (k == key) return true;
+        if (k == kSuperEmpty) return false;
+        b = (b + 1) & mask;
+    }
+    return false;
+}
+__device__ __forceinline__ bool super_occupied_split(const GridView &g, int sx, int sy, int sz) {
+    const unsigned long long key = super_key(sx, sy, sz), k0 = __ldg(g.sbkeys + super_home(key, g.sbmask));
+    bool occ = k0 == key;
+    if (k0 != key && k0 != kSuperEmpty) occ = super_occupied_on(g.sbkeys, g.sbmask, key);
+    return occ;
 }
 
 // floor(u) for |u| < 2^22, from an addition of 1.5 2^23 rounded down; beyond,

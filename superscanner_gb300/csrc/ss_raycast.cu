@@ -43,27 +43,48 @@ __device__ __forceinline__ float floor_and_distance(float p, float rlen, float &
     return fabsf(d);
 }
 
-// idx_rule(a, len) by idx_fast's test where that is decisive (rlen = RN(1 / len)).
-__device__ __forceinline__ int idx_rule_fast(float a, float len, float rlen) {
+// idx_rule(a, len) by idx_fast's test (rlen = RN(1 / len)); false where that is
+// not decisive.
+__device__ __forceinline__ bool idx_sure(float a, float rlen, int &out) {
     float q;
+    const float d = floor_and_distance(a, rlen, q, out);
+    return d > __fmaf_rn(fabsf(q), 3.0e-7f, 3.0e-7f);
+}
+__device__ __forceinline__ int idx_rule_fast(float a, float len, float rlen) {
     int o;
-    const float d = floor_and_distance(a, rlen, q, o);
-    return d > __fmaf_rn(fabsf(q), 3.0e-7f, 3.0e-7f) ? o : idx_rule(a, len);
+    return idx_sure(a, rlen, o) ? o : idx_rule(a, len);
+}
+
+// The rare ways are functions of their own behind one branch each, and what can
+// be selected is selected: a step's time is its chain of instructions and
+// branches, each of which parts a warp and rejoins it (with the voxel loop's and
+// the table finds' likewise 140 -> 125 us with colour and 132 -> 117 without at
+// 640 x 480, 92 -> 80 at 517 x 389, 56 -> 48 at 160 x 120).
+static __device__ __noinline__ int3 idx_slow(float px, float py, float pz, float len) {
+    return make_int3(idx_rule(px, len), idx_rule(py, len), idx_rule(pz, len));
 }
 
 // getVBIndeces (GPUVoxelGrid.h:162-189): the index rule of each coordinate
 // (by multiplication where that is provably the IEEE quotient's result).
 __device__ __forceinline__ void block_of(const GridView &g, F3 p, int &bx, int &by, int &bz) {
-    bx = idx_rule_fast(p.x, g.vbl, g.rvbl);
-    by = idx_rule_fast(p.y, g.vbl, g.rvbl);
-    bz = idx_rule_fast(p.z, g.vbl, g.rvbl);
+    if (!(idx_sure(p.x, g.rvbl, bx) & idx_sure(p.y, g.rvbl, by) & idx_sure(p.z, g.rvbl, bz))) {
+        const int3 b = idx_slow(p.x, p.y, p.z, g.vbl);
+        bx = b.x;
+        by = b.y;
+        bz = b.z;
+    }
 }
 
 // getVinVBIndeces (GPUVoxelGrid.h:192-221): p - vbl * vbInd, then the index rule.
 __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, int by, int bz) {
     const F3 q = f3sub(p, F3{__fmul_rn(g.vbl, (float)bx), __fmul_rn(g.vbl, (float)by), __fmul_rn(g.vbl, (float)bz)});
-    const int vx = idx_rule_fast(q.x, g.vl, g.rvl), vy = idx_rule_fast(q.y, g.vl, g.rvl),
-              vz = idx_rule_fast(q.z, g.vl, g.rvl);
+    int vx, vy, vz;
+    if (!(idx_sure(q.x, g.rvl, vx) & idx_sure(q.y, g.rvl, vy) & idx_sure(q.z, g.rvl, vz))) {
+        const int3 v = idx_slow(q.x, q.y, q.z, g.vl);
+        vx = v.x;
+        vy = v.y;
+        vz = v.z;
+    }
     return vx + kEdge * vy + kEdge * kEdge * vz;
 }
 
@@ -89,17 +110,19 @@ static __device__ __noinline__ int4 voxel_slow(float px, float py, float pz, flo
 }
 __device__ __forceinline__ int voxel_of(const GridView &g, F3 p, int &bx, int &by, int &bz) {
     int x, y, z;
-    if (voxel_fast(p.x, g.rvl, x) & voxel_fast(p.y, g.rvl, y) & voxel_fast(p.z, g.rvl, z)) {
-        bx = x >> 3;
-        by = y >> 3;
-        bz = z >> 3;
-        return (x & 7) + kEdge * (y & 7) + kEdge * kEdge * (z & 7);
+    const bool sure = voxel_fast(p.x, g.rvl, x) & voxel_fast(p.y, g.rvl, y) & voxel_fast(p.z, g.rvl, z);
+    bx = x >> 3;
+    by = y >> 3;
+    bz = z >> 3;
+    int v = (x & 7) + kEdge * (y & 7) + kEdge * kEdge * (z & 7);
+    if (!sure) {
+        const int4 r = voxel_slow(p.x, p.y, p.z, g.vl, g.rvl, g.vbl, g.rvbl);
+        bx = r.x;
+        by = r.y;
+        bz = r.z;
+        v = r.w;
     }
-    const int4 r = voxel_slow(p.x, p.y, p.z, g.vl, g.rvl, g.vbl, g.rvbl);
-    bx = r.x;
-    by = r.y;
-    bz = r.z;
-    return r.w;
+    return v;
 }
 
 // getVoxelMidPoint (GPUVoxelGrid.h:274-278): vb*vbl (float) + (v + 0.5)*vl
@@ -130,13 +153,13 @@ __device__ __forceinline__ int find_block(const GridView &g, int bx, int by, int
             sc.sx = sx;
             sc.sy = sy;
             sc.sz = sz;
-            sc.occ = super_occupied(g, sx, sy, sz);
+            sc.occ = super_occupied_split(g, sx, sy, sz);
             finds++;
         }
         if (!sc.occ) return -1;
     }
     finds++;
-    return table_find(g, prime_hash(bx, by, bz));
+    return table_find_split(g, prime_hash(bx, by, bz));
 }
 
 // The shortest difference between two block coordinates with the same prime
@@ -208,7 +231,8 @@ __global__ void __launch_bounds__(256, 4) raycast_ref_kernel(GridView g, Mat34 E
     // 1.1 ms a call at 640 x 480); every loop's end is one condition instead.
     // 25 of 32 lanes are then active (16.6 before), and a call went from 0.323
     // to 0.19 ms; with the next block's probe issued before the voxel's value is
-    // looked at, and block and voxel from one quotient (voxel_of), to 0.14 ms.
+    // looked at, and block and voxel from one quotient (voxel_of), to 0.14 ms;
+    // with selections for the branches of a step, to 0.12 ms.
     // What is left is the chain of a step's instructions on the longest rays'
     // warps: two voxels a step, the next voxel's value ahead, and four probes
     // of the block skip in flight were slower (0.15, 0.17, 0.15 ms).
@@ -260,31 +284,28 @@ __global__ void __launch_bounds__(256, 4) raycast_ref_kernel(GridView g, Mat34 E
             const int nv = voxel_of(g, nrv, nx, ny, nz);
             const bool same = nx == bx && ny == by && nz == bz;
             // likewise the next block's first probe
-            unsigned long long key = 0, k0 = 0;
-            uint32_t home = 0;
-            if (!same) {
-                key = prime_hash(nx, ny, nz);
-                home = home_bucket(key, g.mask);
-                k0 = __ldg(g.keys + home);
-            }
-            if (cv.w > 0 && !(cv.sdf > 0)) {
-                done = Lp;  // a zero crossing, else a back face
-                Fn = !Lp;
-            } else {
-                Lp = cv.w > 0;
-                rv = nrv;
-                l = __fadd_rn(l, vl);
-                bx = nx;
-                by = ny;
-                bz = nz;
-                v = nv;
-                if (!same && l < dmax) {
-                    finds++;
-                    bucket = k0 == key ? (int)home : k0 == kEmptyKey ? -1 : table_find(g, key);
-                }
-            }
-            in = !done && !Fn && l < dmax && bucket >= 0;
-            if (in) in = ++guard < iter_cap;
+            const unsigned long long key = prime_hash(nx, ny, nz);
+            const uint32_t home = home_bucket(key, g.mask);
+            const unsigned long long k0 = same ? kEmptyKey : __ldg(g.keys + home);
+            const bool cross = cv.w > 0 && !(cv.sdf > 0);
+            done = cross && Lp;  // a zero crossing, else a back face
+            Fn = cross && !Lp;
+            Lp = cross ? Lp : cv.w > 0;
+            rv.x = cross ? rv.x : nrv.x;
+            rv.y = cross ? rv.y : nrv.y;
+            rv.z = cross ? rv.z : nrv.z;
+            l = cross ? l : __fadd_rn(l, vl);
+            bx = cross ? bx : nx;
+            by = cross ? by : ny;
+            bz = cross ? bz : nz;
+            v = cross ? v : nv;
+            const bool look = !cross && !same && l < dmax;
+            finds += look ? 1 : 0;
+            bucket = look ? (k0 == key ? (int)home : -1) : bucket;
+            if (look && k0 != key && k0 != kEmptyKey) bucket = table_find_on(g.keys, g.mask, key);
+            in = !cross && l < dmax && bucket >= 0;
+            guard += in ? 1 : 0;
+            in = in && guard < iter_cap;
         }
         go = go && !done && !Fn && l < dmax && guard < iter_cap;
     }
@@ -551,9 +572,9 @@ extern "C" ss_status ss_raycast(ss_grid *g, const float extr[16], float *ray_pcd
     cudaStream_t s = (cudaStream_t)stream;
     // A warp lasts as long as its longest ray. Where full warps would be no more
     // than four a scheduler, an image ends with its slowest warp, and warps of
-    // half the rays wait for fewer: 56 vs 61 us at 160 x 120, 80 vs 84 at
-    // 320 x 240. Beyond, the second half of the warps costs issue slots: 114 vs
-    // 92 us at 517 x 389, 173 vs 132 at 640 x 480.
+    // half the rays wait for fewer: 48 vs 53 us at 160 x 120, 70 vs 71 at
+    // 320 x 240. Beyond, the second half of the warps costs issue slots: 84 vs
+    // 75 us at 400 x 300, 104 vs 80 at 517 x 389, 160 vs 117 at 640 x 480.
     const int64_t pixels = (int64_t)g->p.resi * g->p.resj;
     const int shift = pixels <= (int64_t)g->num_sms * 4 * 4 * 32 ? 2 : 3;
     const dim3 blk(32, 8), grid((g->p.resj + (4 << shift) - 1) / (4 << shift), (g->p.resi + 7) / 8);

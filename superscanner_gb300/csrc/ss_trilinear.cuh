@@ -50,13 +50,16 @@ __device__ __forceinline__ bool voxel_seen(const GridView &g, int bucket, int v)
     return kStorage == SS_STORAGE_F32 ? __ldg(&g.vox32[vi].y) > 0.f : __ldg(g.vox16 + vi) > 0xFFFFu;
 }
 
+template <bool kSplit = false>
 __device__ __forceinline__ int cached_lookup(const GridView &g, BlockCache &c, int bx, int by, int bz) {
     if (bx == c.x && by == c.y && bz == c.z) return c.bucket;
     c.x = bx;
     c.y = by;
     c.z = bz;
     c.lookups++;
-    c.bucket = packable(bx, by, bz) ? table_find(g, prime_hash(bx, by, bz)) : -1;
+    c.bucket = !packable(bx, by, bz) ? -1
+               : kSplit              ? table_find_split(g, prime_hash(bx, by, bz))
+                                     : table_find(g, prime_hash(bx, by, bz));
     return c.bucket;
 }
 
@@ -239,11 +242,11 @@ __device__ __forceinline__ bool ray_search(const GridView &g, float ox, float oy
                 csx = sx;
                 csy = sy;
                 csz = sz;
-                cocc = super_occupied(g, sx, sy, sz);
+                cocc = kAhead > 0 ? super_occupied_split(g, sx, sy, sz) : super_occupied(g, sx, sy, sz);
                 cache.lookups++;
             }
             const bool empty_super = !cocc;
-            skip = empty_super || cached_lookup(g, cache, bx, by, bz) < 0;
+            skip = empty_super || cached_lookup<(kAhead > 0)>(g, cache, bx, by, bz) < 0;
             if (skip) {
                 // exit of the empty super-block's (or block's) box along the ray
                 const float box = empty_super ? sbl : g.vbl;
