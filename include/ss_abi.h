@@ -341,6 +341,17 @@ ss_status ss_kokkos_icp_noalloc(const uint16_t *d1, const uint16_t *d2, int32_t 
                                 const double ty[16], int32_t icp_type, double txy_out[16],
                                 float *rmse_out, ss_stream_t s);
 
+/* Test hook of kokkosICP's correspondence search (no reference counterpart):
+ * `iteration` (0 .. 9) iterations of the call, then one that writes, for every
+ * pixel of d1, the pixel of d2 that its search chose: its index, plus 2^30
+ * where the pixel's tile was read from global memory (its windows' region did
+ * not fit in shared memory), or -1 without a correspondence, to taps (device,
+ * rows * cols). txy (host) is the transform that iteration searched with, the
+ * top three rows. Synchronises s. */
+ss_status ss_test_icp_taps(const uint16_t *d1, const uint16_t *d2, int32_t rows, int32_t cols, float fx, float fy,
+                           float cx, float cy, const double tx[16], const double ty[16], int32_t icp_type,
+                           int32_t iteration, int32_t *taps, float txy[12], ss_stream_t s);
+
 /* ------------------------------------------------------------------------
  * The per-frame method (no direct reference counterpart: the reference's
  * raycast is nearest-voxel with no normals and no step cap, GPUVoxelGrid.h:377,

@@ -116,6 +116,8 @@ SIGNATURES = {
                             C.POINTER(C.c_float), _p]),
     "ss_kokkos_icp_noalloc": (_st, [_p, _p, _i32, _i32, _f, _f, _f, _f, _D16, _D16, _i32, _D16,
                                     C.POINTER(C.c_float), _p]),
+    "ss_test_icp_taps": (_st, [_p, _p, _i32, _i32, _f, _f, _f, _f, _D16, _D16, _i32, _i32, _p,
+                               C.POINTER(C.c_float), _p]),
     "ss_raycast_maps": (_st, [_p, _F16, _i32, _f, _f, _p, _f, _p, _p, _p]),
     "ss_raycast_loss": (_st, [_p, _D16, _p, _f, _f, _i32, C.POINTER(C.c_double), C.POINTER(C.c_int64), _p, _p]),
     "ss_raycast_loss_grad": (_st, [_p, _D16, _p, _f, _f, _i32, C.POINTER(C.c_double), C.POINTER(C.c_double), _p,

@@ -653,9 +653,14 @@ struct IcpNear {
 };
 constexpr float kIcpMaxD2 = kIcpMaxDist * kIcpMaxDist * 1.0001f;  // above the square of any accepted distance
 
+// The square of a point-to-point tap's distance (kokkosICP.cpp:91), two of its
+// three products fused into the sum. Which of two near-equal taps is the
+// nearer follows from these roundings: with every product rounded, one call in
+// forty at 640 x 480 took another tap somewhere and its transform moved by
+// 1e-7. Two instructions shorter, too (310 -> 302 us a call).
 __device__ __forceinline__ float icp_dist2(const float4 a, F3 px) {
     const F3 d = f3sub(F3{a.x, a.y, a.z}, px);
-    return f3dot(d, d);
+    return fmaf(d.z, d.z, fmaf(d.x, d.x, __fmul_rn(d.y, d.y)));
 }
 
 // Tap t of the second square without the first (20), and of the window
@@ -798,7 +803,7 @@ __device__ __forceinline__ int icp_search_global(const float4 *__restrict__ ya, 
             const float4 a = __ldg(ya + tag);
             const float dist =
                 kType == SS_ICP_POINT_TO_POINT
-                    ? __fsqrt_rn(icp_dist2(a, px))
+                    ? f3len(f3sub(F3{a.x, a.y, a.z}, px))
                     : fabsf(f3dot(f3sub(icp_tap_point(a, __ldg(uv + l), v), px), F3{a.y, a.z, a.w}));
             if (dist < smallest) {
                 smallest = dist;
@@ -878,6 +883,7 @@ __device__ __forceinline__ void icp_stage(float4 *sA, float *su, const float4 *_
 // Pixels by which an iteration widens the region its CTA needed in the
 // iteration before when it stages that region ahead of its wait.
 constexpr int kIcpMargin = 2;
+constexpr int kIcpTapGlobal = 1 << 30;  // ss_test_icp_taps: a tap of a tile read from global memory
 
 // One kokkosICP iteration: Closest Point Kernel (kokkosICP.cpp:69-115) fused
 // with the host sums (:121-171) and, in the last CTA, the rotation update
@@ -905,12 +911,14 @@ constexpr int kIcpMargin = 2;
 // a tap). Point to point: icp_search_point, pixel by pixel.
 // 64 registers (four CTAs per SM; only the rank-deficient fallback of the
 // last CTA spills).
-template <int kType>
+// kTaps (ss_test_icp_taps): the chosen taps go out as well.
+template <int kType, bool kTaps = false>
 __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__restrict__ xp,
                                                            const float4 *__restrict__ ya,
                                                            const float *__restrict__ uv, int rows, int cols, Intr in,
                                                            IcpState *st,
-                                                           int4 *__restrict__ regions, int prestage, IcpOut *out) {
+                                                           int4 *__restrict__ regions, int prestage, IcpOut *out,
+                                                           int *__restrict__ taps) {
     __shared__ float4 sA[kIcpStage];      // target entries
     __shared__ float su[2 * kIcpEdge];    // point to plane: the staged columns' and rows' quotients
     __shared__ float2 red[8][kIcpSums];
@@ -1062,6 +1070,13 @@ __global__ void __launch_bounds__(256, 4) icp_ref_iter_kernel(const float *__res
     } else {
         if (sa) best0 = icp_search_global<kType>(ya, uv, cols, ca_i, ca_j, pa);
         if (sb) best1 = icp_search_global<kType>(ya, uv, cols, cb_i, cb_j, pb);
+    }
+    if (kTaps && j < cols) {
+        auto tap = [&](int best) {
+            return best < 0 ? -1 : staged ? (sr0 + best / sw) * cols + sq0 + best % sw : best | kIcpTapGlobal;
+        };
+        if (i0 < rows) taps[p0] = tap(best0);
+        if (i0 + 1 < rows) taps[p1] = tap(best1);
     }
 
     // this thread's terms as float pairs (values 1..16) and the warp's counts
@@ -1376,14 +1391,10 @@ static void orthonormalize_rotation(double *T) {
         for (int c = 0; c < 3; c++) T[r * 4 + c] = X[r * 3 + c];
 }
 
-// Runs the 10 iterations on prepared point clouds; shared by the entry points.
-// With a host-mapped result (out_host, out_dev) the final iteration writes
-// it there and the call ends with a stream synchronisation; without, the
-// state is copied back.
-ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols, Intr in, const double tx[16],
-                      const double ty[16], int type, float *xp, float4 *ya, float *uv, int ctas,
-                      int4 *regions, IcpState *state, IcpOut *out_host, IcpOut *out_dev, double txy_out[16],
-                      float *rmse_out, cudaStream_t s) {
+// Prepares a call: the point clouds, and the state with Txy = ty^-1 * tx.
+static ss_status icp_prepare(const uint16_t *d1, const uint16_t *d2, int rows, int cols, Intr in, const double tx[16],
+                             const double ty[16], int type, float *xp, float4 *ya, float *uv, IcpState *state,
+                             cudaStream_t s) {
     // Txy = ty^-1 * tx (kokkosICP.cpp:57), float copy for the search
     double tyi[16], T[16];
     inverse4d(ty, tyi);
@@ -1398,28 +1409,39 @@ ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols
     const dim3 blk(128), grid((cols + 127) / 128, rows);
     icp_prep_kernel<<<grid, blk, 0, s>>>(d1, d2, rows, cols, in, type, xp, ya, uv, ini, state);
     SS_LAUNCH_CHECK();
-    const dim3 tiles(icp_tiles_x(cols), icp_tiles_y(rows));  // ctas == tiles.x * tiles.y
-    // four CTAs per SM (64 registers, 38 KB of shared memory each) need the
+    return SS_OK;
+}
+
+// Launches iterations [0, n) of a prepared call; out: the last one's mapped result, or null.
+static ss_status icp_iterate(int rows, int cols, Intr in, int type, const float *xp, const float4 *ya, const float *uv,
+                             int4 *regions, IcpState *state, int n, IcpOut *out, cudaStream_t s) {
+    auto *kernel = type == SS_ICP_POINT_TO_POINT ? icp_ref_iter_kernel<SS_ICP_POINT_TO_POINT>
+                                                 : icp_ref_iter_kernel<SS_ICP_POINT_TO_PLANE>;
+    // four CTAs per SM (64 registers, 27 KB of shared memory each) need the
     // largest shared-memory carveout; a hint, so its status is not fatal
-    if (type == SS_ICP_POINT_TO_POINT)
-        cudaFuncSetAttribute(icp_ref_iter_kernel<SS_ICP_POINT_TO_POINT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
-    else
-        cudaFuncSetAttribute(icp_ref_iter_kernel<SS_ICP_POINT_TO_PLANE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
     cudaGetLastError();
+    const dim3 tiles(icp_tiles_x(cols), icp_tiles_y(rows));
     // programmatic dependent launches: an iteration's CTAs start while the
     // previous one's last CTA forms the transform (not the first: it loads the
     // source points that the launch before it writes before it waits)
-    for (int it = 0; it < kIcpIters; it++) {
-        IcpOut *o = it == kIcpIters - 1 ? out_dev : nullptr;
-        if (type == SS_ICP_POINT_TO_POINT)
-            SS_CUDA_TRY(launch_kernel(icp_ref_iter_kernel<SS_ICP_POINT_TO_POINT>, tiles, dim3(256), 0, s, it > 0, xp, ya,
-                                      uv, rows, cols, in, state, regions, (int)(it > 0), o));
-        else
-            SS_CUDA_TRY(launch_kernel(icp_ref_iter_kernel<SS_ICP_POINT_TO_PLANE>, tiles, dim3(256), 0, s, it > 0, xp, ya,
-                                      uv, rows, cols, in, state, regions, (int)(it > 0), o));
-    }
+    for (int it = 0; it < n; it++)
+        SS_CUDA_TRY(launch_kernel(kernel, tiles, dim3(256), 0, s, it > 0, xp, ya, uv, rows, cols, in, state, regions,
+                                  (int)(it > 0), it == n - 1 ? out : (IcpOut *)nullptr, (int *)nullptr));
+    return SS_OK;
+}
+
+// Runs the 10 iterations; shared by the entry points.
+// With a host-mapped result (out_host, out_dev) the final iteration writes
+// it there and the call ends with a stream synchronisation; without, the
+// state is copied back.
+ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols, Intr in, const double tx[16],
+                      const double ty[16], int type, float *xp, float4 *ya, float *uv, int4 *regions, IcpState *state,
+                      IcpOut *out_host, IcpOut *out_dev, double txy_out[16], float *rmse_out, cudaStream_t s) {
+    ss_status st = icp_prepare(d1, d2, rows, cols, in, tx, ty, type, xp, ya, uv, state, s);
+    if (st != SS_OK) return st;
+    st = icp_iterate(rows, cols, in, type, xp, ya, uv, regions, state, kIcpIters, out_dev, s);
+    if (st != SS_OK) return st;
     float2 best[16];
     float lowest;
     if (out_host) {
@@ -1583,11 +1605,41 @@ ss_status ss_kokkos_icp_noalloc(const uint16_t *d1, const uint16_t *d2, int32_t 
     int4 *regions = (int4 *)(base + kNoAllocImages);
     IcpState *state = (IcpState *)(base + kNoAllocImages + kNoAllocRegions);
     const Intr in{fx, fy, (float)rows - cy, cx};
-    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, xp, ya, uv, ctas, regions, state, nullptr,
+    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, xp, ya, uv, regions, state, nullptr,
                        nullptr, txy_out,
                        rmse_out, (cudaStream_t)stream);
 }
 
+
+ss_status ss_test_icp_taps(const uint16_t *d1, const uint16_t *d2, int32_t rows, int32_t cols, float fx, float fy,
+                           float cx, float cy, const double tx[16], const double ty[16], int32_t icp_type,
+                           int32_t iteration, int32_t *taps, float txy[12], ss_stream_t stream) {
+    if (!taps || !txy || iteration < 0 || iteration >= kIcpIters) return SS_ERR_ARG;
+    double unused[16];
+    ss_status st = icp_check_args(d1, d2, rows, cols, fx, fy, tx, ty, icp_type, unused);
+    if (st != SS_OK) return st;
+    if ((int64_t)rows * cols >= kIcpTapGlobal) return SS_ERR_DIMS;
+    int dev = 0;
+    SS_CUDA_TRY(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(g_icp_mutex);
+    IcpWorkspace *w = nullptr;
+    st = icp_workspace(dev, (size_t)rows * cols, rows + cols, icp_tiles_x(cols) * icp_tiles_y(rows), &w);
+    if (st != SS_OK) return st;
+    const Intr in{fx, fy, (float)rows - cy, cx};
+    cudaStream_t s = (cudaStream_t)stream;
+    st = icp_prepare(d1, d2, rows, cols, in, tx, ty, icp_type, w->xp, w->ya, w->uv, w->state, s);
+    if (st == SS_OK)
+        st = icp_iterate(rows, cols, in, icp_type, w->xp, w->ya, w->uv, w->regions, w->state, iteration, nullptr, s);
+    if (st != SS_OK) return st;
+    SS_CUDA_TRY(cudaMemcpyAsync(txy, w->state->Txy, 12 * sizeof(float), cudaMemcpyDeviceToHost, s));
+    auto *kernel = icp_type == SS_ICP_POINT_TO_POINT ? icp_ref_iter_kernel<SS_ICP_POINT_TO_POINT, true>
+                                                     : icp_ref_iter_kernel<SS_ICP_POINT_TO_PLANE, true>;
+    SS_CUDA_TRY(launch_kernel(kernel, dim3(icp_tiles_x(cols), icp_tiles_y(rows)), dim3(256), 0, s, false,
+                              (const float *)w->xp, (const float4 *)w->ya, (const float *)w->uv, rows, cols, in,
+                              w->state, w->regions, (int)(iteration > 0), (IcpOut *)nullptr, taps));
+    SS_CUDA_TRY(cudaStreamSynchronize(s));
+    return SS_OK;
+}
 
 ss_status ss_depth_to_pcd(const uint16_t *depth, int32_t rows, int32_t cols, float fx, float fy, float cx, float cy,
                           float *pcd, ss_stream_t stream) {
@@ -1618,7 +1670,7 @@ ss_status ss_kokkos_icp(const uint16_t *d1, const uint16_t *d2, int32_t rows, in
     st = icp_workspace(dev, (size_t)rows * cols, rows + cols, ctas, &w);
     if (st != SS_OK) return st;
     const Intr in{fx, fy, (float)rows - cy, cx};  // ci = resi - cy, cj = cx (kokkosICP.cpp:48-49)
-    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, w->xp, w->ya, w->uv, ctas, w->regions,
+    return icp_ref_run(d1, d2, rows, cols, in, tx, ty, icp_type, w->xp, w->ya, w->uv, w->regions,
                        w->state, w->out_host, w->out_dev,
                        txy_out, rmse_out, (cudaStream_t)stream);
 }
