@@ -526,6 +526,13 @@ __device__ __forceinline__ F3 icp_tap_point(const float4 a, float u, float v) {
     return {__fmul_rn(u, a.x), __fmul_rn(v, a.x), a.x};
 }
 
+// A staged point-to-plane tap's distance (kokkosICP.cpp:101-102), two of its
+// three products fused into the sum: icp_scan_row's pairs round it alike.
+__device__ __forceinline__ float icp_plane_dist(const float4 a, float u, float v, F3 px) {
+    const F3 d = f3sub(icp_tap_point(a, u, v), px);
+    return fabsf(fmaf(d.z, a.w, fmaf(d.x, a.y, __fmul_rn(d.y, a.z))));
+}
+
 // The search state of one point-to-plane window: the even and the odd columns
 // keep separate minima (two independent compare chains) with their taps'
 // indices (staged or image indices, increasing in the window's scan order);
@@ -555,10 +562,9 @@ struct IcpBest {
 // vertical pixel pair's windows share nine of their rows): a half row's taps
 // are loaded once, before their comparisons, and each tap's distances
 // (kokkosICP.cpp:101-102) to both source points are evaluated together
-// (packed pairs of the two points' coordinates px, py, pz). The products of the
-// distance are fused into its sum, in the order that the assembler contracted
-// them in when they were written apart (as a sum of rounded products it takes
-// two instructions more a tap).
+// (packed pairs of the two points' coordinates px, py, pz), rounded as
+// icp_plane_dist rounds them (a sum of rounded products takes two instructions
+// more a tap).
 __device__ __forceinline__ void icp_scan_row(const float4 *sA, const float *u, float v, int row, f32x2 px, f32x2 py,
                                              f32x2 pz, bool ua, IcpBest &ba, bool ub, IcpBest &bb) {
 #pragma unroll
@@ -604,10 +610,7 @@ __device__ __forceinline__ int icp_coop_plane(const float4 *sA, const float *su,
             const int t = k + lane;
             if (t < 4 * kIcpSearch * kIcpSearch) {
                 const int r = r0 + t / (2 * kIcpSearch), c = c0 + t % (2 * kIcpSearch);
-                const float4 a = sA[r * sw + c];
-                const F3 y = icp_tap_point(a, su[c], su[kIcpEdge + r]);
-                const F3 d = f3sub(y, p);  // the distance as icp_scan_row rounds it
-                const float dist = fabsf(fmaf(d.z, a.w, fmaf(d.x, a.y, __fmul_rn(d.y, a.z))));
+                const float dist = icp_plane_dist(sA[r * sw + c], su[c], su[kIcpEdge + r], p);
                 if (dist < smallest) {
                     smallest = dist;
                     tap = t;
@@ -790,7 +793,12 @@ __device__ __forceinline__ int icp_search_point(const float4 *sA, bool valid, in
 }
 
 // A window read from global memory (a tile whose window region does not fit
-// the stage): image indices, the reference's loops.
+// the stage): image indices, the reference's loops and its distances with every
+// product rounded (kokkosICP.cpp:91, :101-102). The staged scans fuse two of
+// the products, so of taps whose distances differ by roundings alone the two
+// kinds of tile may take different ones. Neither rounding is brought to the
+// other's tiles: it would move the transform of a call here and there (with
+// the fused one in these tiles 1 of 600 random pairs, by 1.3e-7).
 template <int kType>
 __device__ __forceinline__ int icp_search_global(const float4 *__restrict__ ya, const float *__restrict__ uv, int cols,
                                                  int ci, int cj, F3 px) {

@@ -1,7 +1,8 @@
 """kokkosICP's correspondence searches tap by tap: every pixel's chosen target
 pixel is the one of a full scan of its window with the kernels' roundings (the
-first smallest distance in the reference's order, kokkosICP.cpp:79-113), in
-windows read from shared memory and in those read from global memory."""
+first smallest distance in the reference's order, kokkosICP.cpp:79-113): two of
+a distance's products fused into its sum in windows read from shared memory,
+every product rounded in those read from global memory."""
 import ctypes as C
 
 import numpy as np
@@ -26,7 +27,7 @@ def _fma(a, b, c):
     return _rn32_exact(hi, (p - (hi - v)) + (c - v))
 
 
-def _full_scan(src, dst, normals, T, intr, kind):
+def _full_scan(src, dst, normals, T, intr, kind, fused=True):
     """(tap, the searched pixels, a warp's number of pixels that 16 taps do not settle) by all 100 taps."""
     rows, cols = src.shape[:2]
     fx, fy, cx, cy = (F(v) for v in intr)
@@ -44,13 +45,13 @@ def _full_scan(src, dst, normals, T, intr, kind):
     ti, tj = ci[at][:, None] + k - 5, cj[at][:, None] + l - 5
     t = dst[ti, tj]
     d = t - q[:, None, :]
-    if kind == 0:
-        dist = np.sqrt(_fma(d[..., 2], d[..., 2], _fma(d[..., 0], d[..., 0], d[..., 1] * d[..., 1])))
-        ok = t[..., 2] != 0
+    n = d if kind == 0 else normals[ti, tj]
+    if fused:
+        dot = _fma(d[..., 2], n[..., 2], _fma(d[..., 0], n[..., 0], d[..., 1] * n[..., 1]))
     else:
-        n = normals[ti, tj]
-        dist = np.abs(_fma(d[..., 2], n[..., 2], _fma(d[..., 0], n[..., 0], d[..., 1] * n[..., 1])))
-        ok = (t[..., 2] != 0) & (n[..., 0] != 0)
+        dot = (d[..., 0] * n[..., 0] + d[..., 1] * n[..., 1]) + d[..., 2] * n[..., 2]
+    dist = np.sqrt(dot) if kind == 0 else np.abs(dot)
+    ok = (t[..., 2] != 0) & ((kind == 0) | (n[..., 0] != 0))
     dist = np.where(ok & (dist < F(0.075)), dist, F(np.inf))
     first = dist.argmin(1)
     rng = np.arange(len(first))
@@ -77,10 +78,13 @@ def _taps(d1, d2, tx, kind, intr, iteration):
                                 f64x16(tx), f64x16(np.eye(4)), kind, iteration, C.c_void_p(taps.data_ptr()), txy,
                                 C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     src, dst = (depth_to_pcd(d, *intr) for d in dev)
-    want, inside, more = _full_scan(src.cpu().numpy(), dst.cpu().numpy(), normals_from_pcd(dst).cpu().numpy(),
-                                    np.array(txy[:], F).reshape(3, 4), intr, kind)
+    scene = (src.cpu().numpy(), dst.cpu().numpy(), normals_from_pcd(dst).cpu().numpy(),
+             np.array(txy[:], F).reshape(3, 4), intr, kind)
+    want, inside, more = _full_scan(*scene)
     got = taps.cpu().numpy().astype(np.int64)
     far = (got >= 0) & ((got & GLOBAL) != 0)
+    if far.any():
+        want = np.where(far, _full_scan(*scene, fused=False)[0], want)
     return np.where(far, got & ~GLOBAL, got), want, inside, more, far
 
 
@@ -119,4 +123,22 @@ def test_taps_that_nearly_tie(off, kind):
     tx[:2, 3] = off[0] * 1.5 / 131.3, off[1] * 1.5 / 131.7
     got, want, inside, more, far = _taps(d, d, tx, kind, intr, 0)
     assert inside.sum() > 0.5 * rows * cols and not far.any()
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("rows,cols", [(96, 128), (131, 187)])
+def test_taps_of_tiles_read_from_global_memory(rows, cols, kind):
+    """Patches of two depths, seen from so far aside that the near ones move 0.35 of the image and the far ones a tenth:
+    the windows of a tile lie too far apart for its staged region. Taps nearly tie as in the test above."""
+    f = 0.82 * cols
+    intr = (f, f, (cols - 1) / 2, (rows - 1) / 2)
+    i, j = np.mgrid[0:rows, 0:cols]
+    near = ((i // 8 + j // 8) % 2) == 0
+    d = np.where(near, 700, 2500) if kind == 0 else np.where(near, 700 + j, 2500 + 3 * j)
+    d = d.astype(np.uint16)
+    tx = np.eye(4)
+    tx[:2, 3] = (np.floor(0.35 * cols) + 0.5) * 0.7 / f, 0.5 * 0.7 / f
+    got, want, inside, more, far = _taps(d, d, tx, kind, intr, 0)
+    assert far.sum() > 500
     assert np.array_equal(got, want)
