@@ -38,6 +38,12 @@ struct CellSample {
     int ix, iy, iz; // the cell's lowest voxel
 };
 
+// x . y with its contraction written out: left to the compiler it differs
+// between the forward and the gradient form, and the loss with it.
+__device__ __forceinline__ float dot3(const float x[3], float y0, float y1, float y2) {
+    return fmaf(x[2], y2, fmaf(x[0], y0, __fmul_rn(x[1], y1)));
+}
+
 // Trilinear value, gradient and Hessian of the cell holding p: the corners by
 // the march's own path (all eight loads in flight; the last cell's values
 // kept, and most Newton steps stay in it).
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
 #pragma unroll 1
             for (int it = 0; it < 6 && go; it++) {
                 cell_sample<kStorage>(g, fmaf(t, dx, ox), fmaf(t, dy, oy), fmaf(t, dz, oz), inv_vl, cache, cs);
-                const float gd = cs.g[0] * dx + cs.g[1] * dy + cs.g[2] * dz;
+                const float gd = dot3(cs.g, dx, dy, dz);
                 const float dt = -cs.f / gd;
                 cs.valid = cs.valid && gd < 0.f && !(fabsf(dt) > 2.f * g.vl * inv_len);
                 if (cs.valid) t += dt;
@@ -152,13 +158,14 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
         }
         if (depth_out) depth_out[pix] = cs.valid ? t : 0.f;
         if (cs.valid && d_obs > g.rmin && (!mask || __ldg(mask + pix))) {
-            const float gn = sqrtf(cs.g[0] * cs.g[0] + cs.g[1] * cs.g[1] + cs.g[2] * cs.g[2]);
+            const float gn = sqrtf(dot3(cs.g, cs.g[0], cs.g[1], cs.g[2]));
             const float n[3] = {cs.g[0] / gn, cs.g[1] / gn, cs.g[2] / gn};
             const float d[3] = {dx, dy, dz};
-            const float cdot = n[0] * dx + n[1] * dy + n[2] * dz;
+            const float cdot = dot3(n, dx, dy, dz);
             const float r = t - d_obs;
             if (fabsf(r) < r_max && cdot < -0.05f) {
-                acc[0] = r * r + lambda_n * (r * cdot) * (r * cdot);
+                const float rc = __fmul_rn(r, cdot);
+                acc[0] = fmaf(r, r, __fmul_rn(__fmul_rn(lambda_n, rc), rc));
                 acc[7] = 1.f;
                 if (kBackward) {
                     const float p[3] = {fmaf(t, dx, ox), fmaf(t, dy, oy), fmaf(t, dz, oz)};
