@@ -216,6 +216,14 @@ __device__ __forceinline__ void running_average(float &s, float &w, float obs, f
     }
 }
 
+// min(w, cap) for a weight; a NaN, which only an imported volume holds, stays
+// one, as under running_average's comparison.
+__device__ __forceinline__ float cap_weight(float w, float cap) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(w), "f"(cap));
+    return r;
+}
+
 // The fast update of two voxels at once (the same roundings), weights capped.
 template <bool kDeint, int kStorage>
 __device__ __forceinline__ void running_average_pair(float &s0, float &s1, float &w0, float &w1, f32x2 obs, bool ok0,
@@ -236,11 +244,11 @@ __device__ __forceinline__ void running_average_pair(float &s0, float &s1, float
     }
     if (ok0) {
         s0 = kDeint && v0 == 0.f ? 0.f : a0;
-        w0 = kDeint ? v0 : fminf(v0, cap);
+        w0 = kDeint ? v0 : cap_weight(v0, cap);
     }
     if (ok1) {
         s1 = kDeint && v1 == 0.f ? 0.f : a1;
-        w1 = kDeint ? v1 : fminf(v1, cap);
+        w1 = kDeint ? v1 : cap_weight(v1, cap);
     }
 }
 

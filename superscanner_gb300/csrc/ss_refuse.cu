@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256) refuse_apply_kernel(GridView g, const Ref
                     if (deint)
                         running_average<true, true>(sv, wv, obs[rr], 0.f);
                     else
-                        running_average<false, true>(sv, wv, obs[rr], 0.f), wv = fminf(wv, cap);
+                        running_average<false, true>(sv, wv, obs[rr], 0.f), wv = cap_weight(wv, cap);
                     if (kStorage == SS_STORAGE_F16) {  // the value a sequential call would have stored
                         sv = __half2float(__float2half_rn(sv * inv_trunc)) * g.trunc;
                     }
