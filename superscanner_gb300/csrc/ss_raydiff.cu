@@ -140,8 +140,7 @@ __global__ void __launch_bounds__(256) raydiff_kernel(GridView g, Mat34 T, const
         const float d_obs = (float)__ldg(obs + pix) * 1e-3f;
         pdl_wait();  // the march's hits
         float t = __ldcg(t_hit + pix);
-        CellSample cs;
-        cs.valid = false;
+        CellSample cs{};  // the loop forms its terms from it before it looks at valid
         if (t == t) {  // a hit
             // Newton steps to the root of the trilinear field (bounded, safeguarded)
             bool go = true;
