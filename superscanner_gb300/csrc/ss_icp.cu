@@ -484,6 +484,7 @@ constexpr int kIcpStage = 1536;
 constexpr int kIcpEdge = 160;
 static_assert(kIcpEdge * 10 >= kIcpStage, "a staged region's sides fit the quotient tables");
 constexpr int kIcpSearch = 5;         // n_search (kokkosICP.cpp:53)
+constexpr int kIcpMinSide = 2 * kIcpSearch + 2;  // an image's: room for one window off the border
 constexpr float kIcpMaxDist = 0.075f; // max_dist (kokkosICP.cpp:55)
 constexpr int kIcpCoop = 8;           // up to this many windows of a warp are left to the whole warp, one at a time
 
@@ -1473,7 +1474,7 @@ ss_status icp_ref_run(const uint16_t *d1, const uint16_t *d2, int rows, int cols
 static ss_status icp_check_args(const uint16_t *d1, const uint16_t *d2, int rows, int cols, float fx, float fy,
                                 const double *tx, const double *ty, int type, double *out) {
     if (!d1 || !d2 || !tx || !ty || !out) return SS_ERR_ARG;
-    if (rows <= 2 * 5 + 1 || cols <= 2 * 5 + 1) return SS_ERR_DIMS;
+    if (rows < kIcpMinSide || cols < kIcpMinSide) return SS_ERR_DIMS;
     if (type != SS_ICP_POINT_TO_POINT && type != SS_ICP_POINT_TO_PLANE) return SS_ERR_ARG;
     if (!(fx != 0.f) || !(fy != 0.f)) return SS_ERR_ARG;
     return SS_OK;
@@ -1490,7 +1491,8 @@ constexpr int kNoAllocCtas = 4096;  // iteration-grid CTAs (32 x 16 tiles): any 
 constexpr size_t kAlign256(size_t n) { return (n + 255) / 256 * 256; }
 constexpr size_t kNoAllocSource = kAlign256(kNoAllocMaxPixels * 12);  // source points
 constexpr size_t kNoAllocTarget = kAlign256(kNoAllocMaxPixels * 16);  // target entries
-constexpr size_t kNoAllocSides = kAlign256(kNoAllocMaxPixels * 4);    // column and row quotients (rows + cols <= rows * cols)
+// column and row quotients: both sides are kIcpMinSide or more, so their sum is largest where one is
+constexpr size_t kNoAllocSides = kAlign256((kIcpMinSide + kNoAllocMaxPixels / kIcpMinSide) * sizeof(float));
 constexpr size_t kNoAllocImages = kNoAllocSource + kNoAllocTarget + kNoAllocSides;
 constexpr size_t kNoAllocRegions = kAlign256((size_t)kNoAllocCtas * sizeof(int4));  // staged region per CTA
 constexpr size_t kNoAllocBytes = kNoAllocImages + kNoAllocRegions + kAlign256(sizeof(IcpState));
