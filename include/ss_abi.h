@@ -279,6 +279,22 @@ ss_status ss_grid_test_raycast_cap(ss_grid *g, int32_t cap);
  * SS_ERR_ARG for n < 0 or a value of magnitude 2^47 or more. */
 ss_status ss_test_fixed48_sum(const float *values, int32_t n, double out[3], ss_stream_t s);
 
+/* Test hooks of the kernels' index shortcuts (no reference counterpart), all
+ * arrays on the device, asynchronous on s.
+ * ss_test_voxel_index: for each of n points (x, y, z) the block and the voxel
+ * of a grid of `voxel` metres, eight integers: block x, y, z and the voxel's
+ * index by the raycast's joint rule, then the same by its two separate ones.
+ * ss_test_project: the pixel of each of n (even) coordinates p f / z + c, as
+ * the exact fusion takes it for an image of res pixels.
+ * ss_test_icp_center: for each of n source points under the identity whether
+ * kokkosICP searches for it, and its window's centre row and column (0 where
+ * it does not). */
+ss_status ss_test_voxel_index(const float *points, int32_t n, float voxel, int32_t *out, ss_stream_t s);
+ss_status ss_test_project(const float *p, const float *z, int32_t n, float f, float c, int32_t res, int32_t *out,
+                          ss_stream_t s);
+ss_status ss_test_icp_center(const float *points, int32_t n, int32_t rows, int32_t cols, float fx, float fy, float cx,
+                             float cy, int32_t *out, ss_stream_t s);
+
 /* Text of the last CUDA error seen by this thread (for SS_ERR_CUDA). */
 const char *ss_last_error(void);
 

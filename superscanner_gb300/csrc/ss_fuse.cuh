@@ -25,6 +25,9 @@ static __device__ __noinline__ int project_axis(float p, float f, float z, float
 // for a negative non-integer is one more; past 2^22 the low bits are a number
 // outside any image too. Elsewhere (one coordinate in a thousand at 640 x
 // 480), and for infinities and NaN, the division decides: sure is false.
+__device__ __forceinline__ float project_decide(int res, float c) {
+    return 0.5f - 4.0e-7f * ((float)(res + 2) + fabsf(c));
+}
 __device__ __forceinline__ void project_axis_pair(f32x2 p, float f, f32x2 rz, float c, float decide, int &p0, int &p1,
                                                   bool &sure0, bool &sure1) {
     auto both = [](float v) { return f2_pack(v, v); };
@@ -53,8 +56,7 @@ __device__ __forceinline__ void quad_observe_exact(const GridView &g, const uint
                                                    const Mat34 &Einv, const F3 &Ez, F3 vm0, F3 pz, int l0, int r0,
                                                    float obs[4], bool ok[4], int pix[4]) {
     auto both = [](float v) { return f2_pack(v, v); };
-    const float di = 0.5f - 4.0e-7f * ((float)(g.resi + 2) + fabsf(g.in.ci));
-    const float dj = 0.5f - 4.0e-7f * ((float)(g.resj + 2) + fabsf(g.in.cj));
+    const float di = project_decide(g.resi, g.in.ci), dj = project_decide(g.resj, g.in.cj);
     // the voxels' centres: (vm0.x, y[rr & 1], z[rr >> 1])
     const float y[2] = {vm0.y, __fmaf_rn((float)(l0 + 4) + 0.5f, g.vl, pz.y)};
     const float z[2] = {vm0.z, __fmaf_rn((float)((r0 >> 1) + 1) + 0.5f, g.vl, pz.z)};

@@ -226,8 +226,7 @@ __global__ void __launch_bounds__(256, kColor ? 4 : kExact ? 5 : 8) fuse_kernel(
         int pix4[4];
         if (kExact)
             quad_observe_exact(g, depth, E, Einv, Ez, vm0, F3{pzx, pzy, pzz}, l0, r0, obs4, ok, pix4);
-        else
- {
+        else {
             float ystep[3], zstep[3];
             fast_steps(Einv, g.vl, ystep, zstep);
             f32x2 o[2];
@@ -293,6 +292,23 @@ __global__ void __launch_bounds__(256, kColor ? 4 : kExact ? 5 : 8) fuse_kernel(
 __global__ void finalize_kernel(Counters *ctr) {
     pdl_wait();
     end_call(ctr);
+}
+
+// Test hook kernel: the pixels of pairs of coordinates p f / z + c as quad_observe_exact takes them.
+__global__ void project_pairs_kernel(const float *__restrict__ p, const float *__restrict__ z, int pairs, float f, float c,
+                                     int res, int2 *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= pairs) return;
+    const float p0 = p[2 * k], p1 = p[2 * k + 1], z0 = z[2 * k], z1 = z[2 * k + 1];
+    float r0, r1;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(z0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(z1));
+    int2 i;
+    bool sure0 = true, sure1 = true;
+    project_axis_pair(f2_pack(p0, p1), f, f2_pack(r0, r1), c, project_decide(res, c), i.x, i.y, sure0, sure1);
+    if (!sure0) i.x = project_axis(p0, f, z0, c);
+    if (!sure1) i.y = project_axis(p1, f, z1, c);
+    out[k] = i;
 }
 
 // Clears the epoch field of every stamp (run when the epoch counter wraps).
@@ -640,6 +656,15 @@ ss_status ss_grid_destroy(ss_grid *g) {
     cudaFree(g->t_hit);
     cudaFree(g->batch_phases);
     delete g;
+    return SS_OK;
+}
+
+ss_status ss_test_project(const float *p, const float *z, int32_t n, float f, float c, int32_t res, int32_t *out,
+                          ss_stream_t stream) {
+    if (n < 0 || (n & 1) || (n > 0 && (!p || !z || !out)) || res <= 0) return SS_ERR_ARG;
+    if (n == 0) return SS_OK;
+    project_pairs_kernel<<<(n / 2 + 255) / 256, 256, 0, (cudaStream_t)stream>>>(p, z, n / 2, f, c, res, (int2 *)out);
+    SS_LAUNCH_CHECK();
     return SS_OK;
 }
 

@@ -1523,6 +1523,22 @@ static ss_status noalloc_scratch(int dev, unsigned char **out) {
     return SS_OK;
 }
 
+// Test hook kernel: icp_center of each source point under the identity.
+__global__ void icp_center_kernel(const float *__restrict__ points, int n, int rows, int cols, Intr in,
+                                  int *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    Mat34 T;
+#pragma unroll
+    for (int q = 0; q < 12; q++) T.m[q] = q % 5 == 0 ? 1.f : 0.f;
+    F3 px;
+    int ci, cj;
+    const bool search = icp_center(T, ld3(points, k), in, rows, cols, px, ci, cj);
+    out[3 * k] = search;
+    out[3 * k + 1] = search ? ci : 0;
+    out[3 * k + 2] = search ? cj : 0;
+}
+
 // Test hook kernel: every thread adds its values into the three words; the
 // last CTA (by ticket) forms the total like the kokkosICP and differentiable
 // raycast last CTAs do.
@@ -1620,6 +1636,16 @@ ss_status ss_kokkos_icp_noalloc(const uint16_t *d1, const uint16_t *d2, int32_t 
                        rmse_out, (cudaStream_t)stream);
 }
 
+
+ss_status ss_test_icp_center(const float *points, int32_t n, int32_t rows, int32_t cols, float fx, float fy, float cx,
+                             float cy, int32_t *out, ss_stream_t stream) {
+    if (n < 0 || (n > 0 && (!points || !out)) || rows < kIcpMinSide || cols < kIcpMinSide) return SS_ERR_ARG;
+    if (n == 0) return SS_OK;
+    const Intr in{fx, fy, (float)rows - cy, cx};
+    icp_center_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(points, n, rows, cols, in, out);
+    SS_LAUNCH_CHECK();
+    return SS_OK;
+}
 
 ss_status ss_test_icp_taps(const uint16_t *d1, const uint16_t *d2, int32_t rows, int32_t cols, float fx, float fy,
                            float cx, float cy, const double tx[16], const double ty[16], int32_t icp_type,

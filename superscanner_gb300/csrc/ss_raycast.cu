@@ -589,6 +589,35 @@ extern "C" ss_status ss_raycast(ss_grid *g, const float extr[16], float *ray_pcd
     return SS_OK;
 }
 
+namespace ss {
+// Test hook kernel: block and voxel of each point, by voxel_of and by block_of and voxel_in_block.
+__global__ void voxel_index_kernel(GridView g, const float *__restrict__ points, int n, int4 *__restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const F3 p{points[3 * k], points[3 * k + 1], points[3 * k + 2]};
+    int4 a, b;
+    a.w = voxel_of(g, p, a.x, a.y, a.z);
+    block_of(g, p, b.x, b.y, b.z);
+    b.w = voxel_in_block(g, p, b.x, b.y, b.z);
+    out[2 * k] = a;
+    out[2 * k + 1] = b;
+}
+}  // namespace ss
+
+extern "C" ss_status ss_test_voxel_index(const float *points, int32_t n, float voxel, int32_t *out,
+                                         ss_stream_t stream) {
+    if (n < 0 || (n > 0 && (!points || !out)) || !(voxel > 0.f)) return SS_ERR_ARG;
+    if (n == 0) return SS_OK;
+    GridView g{};
+    g.vl = voxel;
+    g.vbl = 8.f * voxel;
+    g.rvl = 1.f / g.vl;
+    g.rvbl = 1.f / g.vbl;
+    voxel_index_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(g, points, n, (int4 *)out);
+    SS_LAUNCH_CHECK();
+    return SS_OK;
+}
+
 extern "C" ss_status ss_grid_test_raycast_cap(ss_grid *g, int32_t cap) {
     if (!g || cap < 0) return SS_ERR_ARG;
     g->raycast_cap = cap;
