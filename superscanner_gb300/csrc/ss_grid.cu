@@ -670,6 +670,16 @@ ss_status ss_test_project(const float *p, const float *z, int32_t n, float f, fl
 
 ss_status ss_grid_set_intrinsic(ss_grid *g, float fx, float fy, float cx, float cy) {
     if (!g || !(fx != 0.f) || !(fy != 0.f)) return SS_ERR_ARG;
+    if (g->intr_set && fx == g->fx && fy == g->fy && cx == g->cx && cy == g->cy) return SS_OK;
+    // kernels of earlier calls, on whatever stream, read the tables that the
+    // copies below overwrite (those wait for blocking streams alone)
+    int dev = 0;
+    SS_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev != g->device) SS_CUDA_TRY(cudaSetDevice(g->device));
+    const cudaError_t idle = cudaDeviceSynchronize();
+    if (dev != g->device) cudaSetDevice(dev);
+    SS_CUDA_TRY(idle);
+    g->intr_set = false;  // until the tables hold the new quotients
     g->fx = fx;
     g->fy = fy;
     g->cx = cx;
