@@ -695,6 +695,7 @@ ss_status ss_grid_set_intrinsic(ss_grid *g, float fx, float fy, float cx, float 
     SS_CUDA_TRY(cudaMemcpy((void *)g->v.ray_u, u.data(), u.size() * sizeof(float), cudaMemcpyHostToDevice));
     SS_CUDA_TRY(cudaMemcpy((void *)g->v.ray_v, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice));
     g->intr_set = true;
+    g->launch_gen++;  // captured frames hold the old intrinsics
     return SS_OK;
 }
 

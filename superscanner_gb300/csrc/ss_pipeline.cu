@@ -305,7 +305,7 @@ ss_status ss_pipeline_frame(ss_pipeline *P, const uint16_t *depth, int32_t track
         }
     }
     const uint16_t *in = P->inbuf[b];
-    if (P->lc_gen != g->launch_gen) {  // launch shapes changed: new tracker grid, graphs recaptured below
+    if (P->lc_gen != g->launch_gen) {  // launch shapes or intrinsics changed: new tracker grid, graphs recaptured below
         P->track_ctas = persistent_track_ctas(g->num_sms, g->lc.track_ctas_per_sm);
         P->lc_gen = g->launch_gen;
     }
@@ -317,7 +317,7 @@ ss_status ss_pipeline_frame(ss_pipeline *P, const uint16_t *depth, int32_t track
         if (st != SS_OK) return st;
         P->have_model = true;
     } else if (P->p.use_graph && P->test_wait_polls == 0) {
-        if (P->exec[b] && P->exec_gen[b] != g->launch_gen) {  // launch shapes changed since the capture
+        if (P->exec[b] && P->exec_gen[b] != g->launch_gen) {  // launch shapes or intrinsics changed since the capture
             cudaGraphExecDestroy(P->exec[b]);
             cudaGraphDestroy(P->graph[b]);
             P->exec[b] = nullptr;

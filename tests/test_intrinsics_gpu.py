@@ -49,3 +49,31 @@ def test_new_intrinsics_wait_for_calls_in_flight(exact):
         g.close()
     for k in ("keys", "coords", "sdf", "w"):
         assert np.array_equal(out[0][k], out[1][k])
+
+
+@pytest.mark.parametrize("exact", [True, False])
+def test_a_captured_frame_takes_new_intrinsics(exact):
+    """The per-frame graph, captured before the intrinsics changed, against frames launched one by one."""
+    from superscanner_gb300.pipeline import Pipeline
+    P, dev = _scene(6)
+    out = []
+    for graph in (False, True):
+        g = _grid("f16")
+        pipe = Pipeline(g, use_graph=graph, persistent_track=False, exact_fusion=exact)
+        pipe.set_pose(P[0])
+        pipe.frame(dev[0], track=False)
+        pipe.frame(dev[1])
+        pipe.frame(dev[2])
+        torch.cuda.synchronize()
+        g.setIntrinsic(*OTHER)
+        poses = []
+        for k in (3, 4, 5):
+            pipe.frame(dev[k])
+            poses.append(pipe.pose())
+        maps = pipe.maps_tensors()
+        g.sync()
+        out.append((np.stack(poses), *(m.cpu().numpy() for m in maps), *g.export_blocks(with_color=False).values()))
+        pipe.close()
+        g.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b) if a is not None else b is None
