@@ -279,7 +279,7 @@ ss_status ss_grid_test_raycast_cap(ss_grid *g, int32_t cap);
  * SS_ERR_ARG for n < 0 or a value of magnitude 2^47 or more. */
 ss_status ss_test_fixed48_sum(const float *values, int32_t n, double out[3], ss_stream_t s);
 
-/* Test hooks of the kernels' index shortcuts (no reference counterpart), all
+/* Test hooks of the kernels' index rules (no reference counterpart), all
  * arrays on the device, asynchronous on s.
  * ss_test_voxel_index: for each of n points (x, y, z) the block and the voxel
  * of a grid of `voxel` metres, eight integers: block x, y, z and the voxel's

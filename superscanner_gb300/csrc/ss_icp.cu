@@ -488,36 +488,14 @@ constexpr int kIcpMinSide = 2 * kIcpSearch + 2;  // an image's: room for one win
 constexpr float kIcpMaxDist = 0.075f; // max_dist (kokkosICP.cpp:55)
 constexpr int kIcpCoop = 8;           // up to this many windows of a warp are left to the whole warp, one at a time
 
-static __device__ __noinline__ int2 icp_center_slow(F3 px, Intr in) {
-    return make_int2(__float2int_rz(__fadd_rn(__fdiv_rn(__fmul_rn(px.y, in.fy), px.z), in.ci)),
-                     __float2int_rz(__fadd_rn(__fdiv_rn(__fmul_rn(px.x, in.fx), px.z), in.cj)));
-}
-
 // The transformed source point px = Txy x and its window centre
 // (kokkosICP.cpp:72-76); true when the reference searches (x.z != 0 and the
 // window inside the image, :79).
-// The casts' coordinates come from an approximate reciprocal where that decides
-// them, by the rule of project_axis_pair (ss_fuse.cuh; past the image both lie
-// outside the window's bounds), else from the divisions behind one branch (two
-// inlined divisions a pixel: 163 -> 160 us a call at 160 x 120, 286 -> 282 at
-// 640 x 480, point to point 125 -> 121 at 160 x 120).
 __device__ __forceinline__ bool icp_center(const Mat34 &T, F3 x, Intr in, int rows, int cols, F3 &px, int &ci,
                                            int &cj) {
     px = xform(T, x);
-    float rz;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rz) : "f"(px.z));
-    auto sure = [&](float p, float f, float c, int res, int &out) {
-        const float a = fmaf(__fmul_rn(p, f), rz, c), s = __fadd_rd(a, 12582912.f);
-        out = (int)(__float_as_uint(s) - 0x4B400000u);
-        out += (int)((unsigned)out >> 31);
-        return fabsf(__fsub_rn(__fsub_rn(a, __fsub_rn(s, 12582912.f)), 0.5f)) <
-               0.5f - 4.0e-7f * ((float)(res + 2) + fabsf(c));
-    };
-    if (!(sure(px.y, in.fy, in.ci, rows, ci) & sure(px.x, in.fx, in.cj, cols, cj)) && x.z != 0) {
-        const int2 c = icp_center_slow(px, in);
-        ci = c.x;
-        cj = c.y;
-    }
+    ci = __float2int_rz(__fadd_rn(__fdiv_rn(__fmul_rn(px.y, in.fy), px.z), in.ci));
+    cj = __float2int_rz(__fadd_rn(__fdiv_rn(__fmul_rn(px.x, in.fx), px.z), in.cj));
     return x.z != 0 && ci > kIcpSearch && ci < rows - kIcpSearch && cj > kIcpSearch && cj < cols - kIcpSearch;
 }
 

@@ -1,4 +1,4 @@
-"""The kernels' index shortcuts on the device, against the reference's rules in
+"""The kernels' index rules on the device, against the reference's in
 IEEE single precision, exactly: block and voxel of a point (voxel_of, block_of,
 voxel_in_block), a projected voxel's pixel (project_axis_pair), a kokkosICP
 window's centre (icp_center). Points next to every boundary, negative ones, past
