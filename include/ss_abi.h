@@ -102,7 +102,9 @@ ss_status ss_grid_set_launch_config(ss_grid *g, const ss_launch_config *c);
 ss_status ss_grid_reset(ss_grid *g, ss_stream_t s);
 
 /* setIntrinsic (GPUVoxelGrid.cpp:253-266): fx, fy, cx, cy of the pinhole model;
- * the grid uses ci = resi - cy, cj = cx exactly as the reference. */
+ * the grid uses ci = resi - cy, cj = cx exactly as the reference. Where they
+ * change it waits for the device (calls in flight use the old ones), and
+ * captured per-frame graphs are re-captured. */
 ss_status ss_grid_set_intrinsic(ss_grid *g, float fx, float fy, float cx, float cy);
 
 /* integrate / deIntegrate (GPUVoxelGrid.cpp:41-136). depth: [resi][resj] u16 mm,

@@ -637,9 +637,9 @@ constexpr float kIcpMaxD2 = kIcpMaxDist * kIcpMaxDist * 1.0001f;  // above the s
 
 // The square of a point-to-point tap's distance (kokkosICP.cpp:91), two of its
 // three products fused into the sum. Which of two near-equal taps is the
-// nearer follows from these roundings: with every product rounded, one call in
-// forty at 640 x 480 took another tap somewhere and its transform moved by
-// 1e-7. Two instructions shorter, too (310 -> 302 us a call).
+// nearer follows from these roundings: with every product rounded, 1 of 40
+// pairs of 640 x 480 took another tap somewhere and its transform moved by
+// 1.8e-7. Two instructions shorter, too (310 -> 302 us a call).
 __device__ __forceinline__ float icp_dist2(const float4 a, F3 px) {
     const F3 d = f3sub(F3{a.x, a.y, a.z}, px);
     return fmaf(d.z, d.z, fmaf(d.x, d.x, __fmul_rn(d.y, d.y)));
