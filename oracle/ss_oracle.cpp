@@ -25,7 +25,7 @@
 // conversion the reference actually ran (truncate toward zero, saturate,
 // NaN -> 0), see f2i() below.
 //
-// Four behaviours of the reference are data races or undefined; the oracle
+// Three behaviours of the reference are data races or undefined; the oracle
 // and the CUDA path share one canonical resolution for each:
 //  * Blocks whose prime hashes collide alias one map entry and the entry's
 //    pzero/vbInd are written by every visitor (GPUVoxelGrid.cpp:500-502, last
@@ -35,10 +35,6 @@
 //    the reference calls value_at(find(..)) on an invalid index
 //    (GPUVoxelGrid.cpp:669-672). Canonical rule: that voxel reads as empty
 //    (w = 0, sdf = 0, colour 0).
-//  * The raycast's index rules can give a voxel axis 8 or -1 next to a block's
-//    face (getVinVBIndeces, GPUVoxelGrid.h:192-221: at a negative multiple of
-//    the block's edge, say), and with it a linear index outside the block's
-//    512. Canonical rule: each axis takes its nearest voxel then.
 //  * kokkosICP's correspondence view is never zeroed before the first
 //    iteration (kokkosICP.cpp:43; Kvec3f's default constructor,
 //    kokkosFunctions.h:149, writes nothing), so pixels without a
@@ -486,12 +482,7 @@ void orc_grid_raycast(void *h, const float *Er, float *ray_pcd, float *ray_color
             };
             auto vin_of = [&](V3 p, I3 b) {
                 V3 q = sub(p, V3{vbl * b.x, vbl * b.y, vbl * b.z});
-                I3 v{idx_rule(q.x, vl), idx_rule(q.y, vl), idx_rule(q.z, vl)};
-                if ((unsigned)v.x + kEdge * (unsigned)v.y + kEdge * kEdge * (unsigned)v.z >= kEdge * kEdge * kEdge) {
-                    auto in = [](int a) { return a < 0 ? 0 : a >= kEdge ? kEdge - 1 : a; };
-                    v = I3{in(v.x), in(v.y), in(v.z)};
-                }
-                return v;
+                return I3{idx_rule(q.x, vl), idx_rule(q.y, vl), idx_rule(q.z, vl)};
             };
             auto mid = [&](I3 v, I3 b) {  // getVoxelMidPoint (GPUVoxelGrid.h:274-278)
                 return V3{(float)(b.x * vbl + (v.x + 0.5) * vl), (float)(b.y * vbl + (v.y + 0.5) * vl),

@@ -75,18 +75,6 @@ __device__ __forceinline__ void block_of(const GridView &g, F3 p, int &bx, int &
     }
 }
 
-// A voxel's place in its block of 512. Next to a block's face the reference's
-// rules can give an axis 8 or -1 (at a negative multiple of the block's edge;
-// where the point's distance to the face is lost in its rounding), and so a
-// place outside the block, where the reference reads whatever lies there. Each
-// axis takes its nearest voxel then.
-__device__ __forceinline__ int voxel_place(int vx, int vy, int vz) {
-    unsigned v = (unsigned)vx + kEdge * (unsigned)vy + kEdge * kEdge * (unsigned)vz;
-    if (v >= kBlockVoxels)
-        v = min(max(vx, 0), kEdge - 1) + kEdge * min(max(vy, 0), kEdge - 1) + kEdge * kEdge * min(max(vz, 0), kEdge - 1);
-    return (int)v;
-}
-
 // getVinVBIndeces (GPUVoxelGrid.h:192-221): p - vbl * vbInd, then the index rule.
 __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, int by, int bz) {
     const F3 q = f3sub(p, F3{__fmul_rn(g.vbl, (float)bx), __fmul_rn(g.vbl, (float)by), __fmul_rn(g.vbl, (float)bz)});
@@ -97,7 +85,7 @@ __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, i
         vy = v.y;
         vz = v.z;
     }
-    return voxel_place(vx, vy, vz);
+    return vx + kEdge * vy + kEdge * kEdge * vz;
 }
 
 // Block and voxel of a point at once (block_of, then voxel_in_block). With
@@ -118,7 +106,7 @@ static __device__ __noinline__ int4 voxel_slow(float px, float py, float pz, flo
     const int bx = idx_rule_fast(px, vbl, rvbl), by = idx_rule_fast(py, vbl, rvbl), bz = idx_rule_fast(pz, vbl, rvbl);
     const F3 q = f3sub(F3{px, py, pz}, F3{__fmul_rn(vbl, (float)bx), __fmul_rn(vbl, (float)by), __fmul_rn(vbl, (float)bz)});
     const int vx = idx_rule_fast(q.x, vl, rvl), vy = idx_rule_fast(q.y, vl, rvl), vz = idx_rule_fast(q.z, vl, rvl);
-    return make_int4(bx, by, bz, voxel_place(vx, vy, vz));
+    return make_int4(bx, by, bz, vx + kEdge * vy + kEdge * kEdge * vz);
 }
 __device__ __forceinline__ int voxel_of(const GridView &g, F3 p, int &bx, int &by, int &bz) {
     int x, y, z;
