@@ -521,6 +521,22 @@ ss_status launch_fuse(ss_grid *g, const uint16_t *depth, const uint8_t *rgb, con
 
 using namespace ss;
 
+// An array of B blocks of n elements with an empty block before its first and
+// one behind its last: the raycast's index rules can name a place next to its
+// block (voxel_place, ss_raycast.cu).
+template <class T>
+static bool alloc_blocks(T **out, size_t B, size_t n) {
+    T *base = nullptr;
+    if (cudaMalloc(&base, (B + 2) * n * sizeof(T)) != cudaSuccess) return false;
+    *out = base + n;
+    return cudaMemset(base, 0, n * sizeof(T)) == cudaSuccess &&
+           cudaMemset(base + (B + 1) * n, 0, n * sizeof(T)) == cudaSuccess;
+}
+template <class T>
+static void free_blocks(T *blocks, size_t n) {
+    if (blocks) cudaFree(blocks - n);
+}
+
 extern "C" {
 
 const char *ss_last_error(void) { return g_last_error.c_str(); }
@@ -608,11 +624,9 @@ ss_status ss_grid_create(const ss_params *p, ss_grid **out) {
     const size_t SB = std::max<size_t>(4096, B);
     if (ok) ok = cudaMalloc(&g->v.sbkeys, SB * 8) == cudaSuccess;
     g->v.sbmask = (uint32_t)(SB - 1);
-    if (ok && p->storage == SS_STORAGE_F32)
-        ok = cudaMalloc(&g->v.vox32, B * kBlockVoxels * sizeof(float2)) == cudaSuccess;
-    if (ok && p->storage == SS_STORAGE_F16)
-        ok = cudaMalloc(&g->v.vox16, B * kBlockVoxels * sizeof(uint32_t)) == cudaSuccess;
-    if (ok && p->with_color) ok = cudaMalloc(&g->v.rgb, B * 3 * kBlockVoxels * sizeof(float)) == cudaSuccess;
+    if (ok && p->storage == SS_STORAGE_F32) ok = alloc_blocks(&g->v.vox32, B, kBlockVoxels);
+    if (ok && p->storage == SS_STORAGE_F16) ok = alloc_blocks(&g->v.vox16, B, kBlockVoxels);
+    if (ok && p->with_color) ok = alloc_blocks(&g->v.rgb, B, 3 * kBlockVoxels);
     if (!ok) {
         cudaGetLastError();
         ss_grid_destroy(g);
@@ -645,9 +659,9 @@ ss_status ss_grid_destroy(ss_grid *g) {
     cudaFree(g->v.stamp);
     cudaFree(g->v.list);
     cudaFree(g->v.ctr);
-    cudaFree(g->v.vox32);
-    cudaFree(g->v.vox16);
-    cudaFree(g->v.rgb);
+    free_blocks(g->v.vox32, kBlockVoxels);
+    free_blocks(g->v.vox16, kBlockVoxels);
+    free_blocks(g->v.rgb, 3 * kBlockVoxels);
     cudaFree(g->v.sbkeys);
     cudaFree((void *)g->v.ray_u);
     cudaFree((void *)g->v.ray_v);

@@ -106,6 +106,7 @@ __device__ __forceinline__ void load_pose(const FramePose *p, Mat34 &E, Mat34 &E
 struct GridView {
     unsigned long long *keys;   // [buckets] u64 prime-hash keys
     unsigned long long *stamp;  // [buckets] epoch | packed block coords
+    // an empty block lies before the first bucket's and behind the last's
     float2 *vox32;              // [buckets][512] (sdf, w)     SS_STORAGE_F32
     uint32_t *vox16;            // [buckets][512] half(sdf/trunc) | u16 w << 16   SS_STORAGE_F16
     float *rgb;                 // [buckets][3][512] or null

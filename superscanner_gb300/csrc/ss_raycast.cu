@@ -75,6 +75,21 @@ __device__ __forceinline__ void block_of(const GridView &g, F3 p, int &bx, int &
     }
 }
 
+// A voxel's place in its block of 512. Next to a block's face the reference's
+// rules can give an axis 8 or -1 (at a negative multiple of the block's edge;
+// where the point's distance to the face is lost in its rounding; one pixel of
+// ten frames of a room), and so a place up to 73 voxels before the block or 72
+// behind it, where the reference reads on in whatever lies there. The grid's
+// arrays hold an empty block on either side (ss_grid_create), so such a read
+// stays in them; an axis further out (a point too far from the origin for its
+// block's voxels) takes its nearest voxel.
+__device__ __forceinline__ int voxel_place(int vx, int vy, int vz) {
+    const int v = (int)((unsigned)vx + kEdge * (unsigned)vy + kEdge * kEdge * (unsigned)vz);
+    if (v >= -kBlockVoxels && v < 2 * kBlockVoxels) return v;
+    auto in = [](int a) { return min(max(a, 0), kEdge - 1); };
+    return in(vx) + kEdge * in(vy) + kEdge * kEdge * in(vz);
+}
+
 // getVinVBIndeces (GPUVoxelGrid.h:192-221): p - vbl * vbInd, then the index rule.
 __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, int by, int bz) {
     const F3 q = f3sub(p, F3{__fmul_rn(g.vbl, (float)bx), __fmul_rn(g.vbl, (float)by), __fmul_rn(g.vbl, (float)bz)});
@@ -85,7 +100,7 @@ __device__ __forceinline__ int voxel_in_block(const GridView &g, F3 p, int bx, i
         vy = v.y;
         vz = v.z;
     }
-    return vx + kEdge * vy + kEdge * kEdge * vz;
+    return voxel_place(vx, vy, vz);
 }
 
 // Block and voxel of a point at once (block_of, then voxel_in_block). With
@@ -106,7 +121,7 @@ static __device__ __noinline__ int4 voxel_slow(float px, float py, float pz, flo
     const int bx = idx_rule_fast(px, vbl, rvbl), by = idx_rule_fast(py, vbl, rvbl), bz = idx_rule_fast(pz, vbl, rvbl);
     const F3 q = f3sub(F3{px, py, pz}, F3{__fmul_rn(vbl, (float)bx), __fmul_rn(vbl, (float)by), __fmul_rn(vbl, (float)bz)});
     const int vx = idx_rule_fast(q.x, vl, rvl), vy = idx_rule_fast(q.y, vl, rvl), vz = idx_rule_fast(q.z, vl, rvl);
-    return make_int4(bx, by, bz, vx + kEdge * vy + kEdge * kEdge * vz);
+    return make_int4(bx, by, bz, voxel_place(vx, vy, vz));
 }
 __device__ __forceinline__ int voxel_of(const GridView &g, F3 p, int &bx, int &by, int &bz) {
     int x, y, z;

@@ -50,7 +50,11 @@ def test_block_and_voxel_of_a_point(length):
         vbl = F(8) * vl
         b = _rule(p, vbl)
         v = _rule(p - vbl * b.astype(F), vl)
-        want = np.concatenate([b, (v[:, :1] + 8 * v[:, 1:2] + 64 * v[:, 2:3]).astype(np.int32)], -1)
+        # next to a block's face the rules can give an axis 8 or -1, and a place next to the block; further out: the nearest
+        place = (v.astype(np.uint32) @ np.uint32([1, 8, 64])).view(np.int32)
+        near = np.clip(v, 0, 7) @ np.int32([1, 8, 64])
+        want = np.concatenate([b, np.where((place >= -512) & (place < 1024), place, near)[:, None]], -1)
+    assert ((place < 0) | (place >= 512)).sum() > 1000
     got = out.cpu().numpy()
     assert np.array_equal(got[:, 1], want)
     assert np.array_equal(got[:, 0], want)
